@@ -377,18 +377,27 @@ static int entry_skew_k(const wg_batch *b, const BatchSlotHost &h)
     return b->skew_mode > 0 ? b->skew_mode : b->class_k[h.cls];
 }
 
+// the kernel form that covers every scene of a list: the masked one, or the general one
+static int list_form(const std::vector<const BatchSlotHost *> &hs)
+{
+    int form = hs.empty() ? 0 : batch_skew_form(hs[0]->prm);
+    for (const BatchSlotHost *h : hs)
+        if (batch_skew_form(h->prm) != form) return 0;
+    return form;
+}
+
 // Tasks of the pass depth d for the scenes of depth class K (table entries), largest first
 // so that the ticket order balances the warps.  Row chunks: the rows tuned for the scene's
 // size class, or (untuned, fixed depth) sized from the whole list's work, about two tasks
-// per resident warp (at least 32 rows), so that no single chunk outlasts the rest of the
+// per resident team (at least 32 rows), so that no single chunk outlasts the rest of the
 // pass; the short top and bottom segments fill the end.  force_rows > 0 overrides both.
 static void build_skew_tasks(const wg_batch *b, const std::vector<const BatchSlotHost *> &hs,
                              const std::vector<int> &entries, int d, std::vector<int4> &out, int force_rows = 0)
 {
-    const int F = 2 * d + 1;
+    const int F = batch_skew_fill(d);
     double rows = 0.0;
     for (const BatchSlotHost *h : hs) rows += (double)batch_skew_tiles(h->dp, d) * (h->prm.nx + 3 * F);
-    const int cap = std::max(1, batch_skew_capacity(d));
+    const int cap = std::max(1, batch_skew_capacity(d, list_form(hs)));
     const int chunk = std::max(32, std::min(4096, (int)(rows / (2.0 * cap))));
     std::vector<int4> t;
     std::vector<float> cost;
@@ -432,6 +441,11 @@ static wg_status build_list(wg_batch *b, int K, int d, const std::vector<int> &t
         WG_CUDA(cudaMalloc(&L.dev, sizeof(int4) * cap));
         L.cap = cap;
         batch_drop_graphs(b);  // the graphs hold the list pointer
+    }
+    const int form = list_form(hs);
+    if (form != L.form) {  // the graphs hold the kernel
+        L.form = form;
+        batch_drop_graphs(b);
     }
     L.n = (int)tasks.size();
     if (L.n) WG_CUDA(cudaMemcpyAsync(L.dev, tasks.data(), sizeof(int4) * L.n, cudaMemcpyHostToDevice, b->st));
@@ -569,11 +583,11 @@ static wg_status batch_prepare_frame(wg_batch *b, int n, bool skewed)
         tickets += P;
         for (int q = 0; q < P; q++) {
             const int d = batch_pass_depth(n, P, q);
-            batch_skew_capacity(d);  // sets the kernel's shared-memory attribute outside the capture
             if (!b->lists.count({K, d})) {
                 wg_status st = build_list(b, K, d, b->tab_slot);
                 if (st) return st;
             }
+            batch_skew_capacity(d, b->lists.at({K, d}).form);  // sets the kernel's shared-memory attribute outside the capture
         }
     }
     if (tickets > b->ticket_cap) {
@@ -614,7 +628,7 @@ static void batch_enqueue_frame(wg_batch *b, int n, bool skewed)
                 const BatchSkewList &L = b->lists.at({K, d});
                 if (b->graph_sig & (1u << 8))  // the wrapped scenes' ghosts of this pass's input pair
                     k_batch_ghosts<<<dim3(std::max(b->tab_cap, 1), 8), 256, 0, ss>>>(b->d_hdr, b->d_tab, b->d_dyn, K, q);
-                launch_batch_skew(d, b->d_tab, b->d_dyn, L.dev, b->d_skew_n + L.index, b->d_ticket + ti++, q, toff, ss);
+                launch_batch_skew(d, L.form, b->d_tab, b->d_dyn, L.dev, b->d_skew_n + L.index, b->d_ticket + ti++, q, toff, ss);
                 toff += d;
             }
             cudaEventRecord(b->ev_join[K], ss);
@@ -662,6 +676,7 @@ static unsigned class_kinds(const wg_batch *b, int c)
         if (h.prm.twospeeds) sig |= 1u << 9;
         if (h.prm.oscillate_left || h.prm.oscillate_topbot) sig |= 1u << 10;
         if (h.prm.src_on) sig |= 1u << 11;
+        if (batch_skew_form(h.prm) == 0) sig |= 1u << 12;
     }
     return sig;
 }
@@ -710,9 +725,7 @@ static wg_status batch_autotune(wg_batch *b)
         int4 *dev = nullptr;
         cudaError_t err = cudaSuccess;
         static const int ROWS[] = {32, 64, 128, 256};
-        // depths 2..4: at 5 and 6 the velocity rows push the pass past its 128 registers
-        // (spills) and those depths measured slower on every size class tried
-        const int ndepth = 3;
+        const int ndepth = 5;  // depths 2..6
         for (int cand = 0; cand < ndepth + 4 && err == cudaSuccess; cand++) {
             const int K = cand < ndepth ? 2 + cand : best, R = cand < ndepth ? 0 : ROWS[cand - ndepth];
             std::vector<int4> tasks;
@@ -725,7 +738,7 @@ static wg_status batch_autotune(wg_batch *b)
             const int reps = 5;  // one untimed pass, then the best of five
             for (int r = 0; r <= reps && err == cudaSuccess; r++) {
                 cudaMemsetAsync(b->d_tune_ticket + r, 0, sizeof(int), b->st);
-                launch_batch_skew(K, b->d_tab, b->d_dyn, dev, b->d_skew_n + idx, b->d_tune_ticket + r, 0, 0, b->st);
+                launch_batch_skew(K, list_form(hs), b->d_tab, b->d_dyn, dev, b->d_skew_n + idx, b->d_tune_ticket + r, 0, 0, b->st);
                 b->launches++;
                 err = cudaGetLastError();
                 if (err == cudaSuccess) err = cudaEventRecord(ev[r], b->st);

@@ -58,15 +58,19 @@ __host__ __device__ inline int batch_passes(int n, int K)
 }
 __host__ __device__ inline int batch_pass_depth(int n, int P, int q) { return n / P + (q < n % P ? 1 : 0); }
 
-// Skewed passes over many scenes (wg_tb.cu): persistent warps take tasks (table entry,
+// Skewed passes over many scenes (wg_tb.cu): persistent teams of warps take tasks (table entry,
 // first column of the 128-column tile, rows i_s | i_e << 16, kind) from a ticket counter;
 // pass q of a frame reads the pair the previous pass wrote, toff updates after the frame start.
-int batch_skew_capacity(int K);
+// form: the update its kernel compiles (batch_skew_form: a list of scenes that are all masked
+// takes PL_MASKED, any other list the general form)
+int batch_skew_form(const wg_params &p);
+int batch_skew_capacity(int K, int form);         // resident teams
+int batch_skew_fill(int K);                       // rows a chunk's pipeline fill costs
 int batch_skew_tiles(const DevParams &p, int K);  // column tiles of a scene (shifted tiling)
 // tasks of one scene, inner row chunks of rows..2*rows rows
 void batch_skew_plan(const DevParams &p, int entry, int K, int rows, std::vector<int4> &tasks, std::vector<float> &cost);
-void launch_batch_skew(int K, const SlotDev *tab, const SlotDyn *dyn, const int4 *tasks, const int *ntasks, int *ticket,
-                       int q, int toff, cudaStream_t st);
+void launch_batch_skew(int K, int form, const SlotDev *tab, const SlotDyn *dyn, const int4 *tasks, const int *ntasks,
+                       int *ticket, int q, int toff, cudaStream_t st);
 bool batch_skew_ok(const wg_params &p, int prec);
 bool batch_wrap_ok(const wg_params &p, int prec);   // periodic scenes the skewed passes take (ghost layout)
 
@@ -100,6 +104,7 @@ struct BatchSlotHost {
 struct BatchSkewList {      // tasks of one pass depth for one depth class
     int4 *dev = nullptr;
     int cap = 0, n = 0, index = 0;  // index: its count in d_skew_n
+    int form = -1;                  // the kernel form of its scenes (batch_skew_form)
 };
 
 struct wg_batch {
