@@ -1,14 +1,14 @@
 // wg_batch.cu — many scenes of uneven sizes advanced together.
 //
-// Single updates: every active scene is cut into work items of BT_ROWS rows x (64
-// threads x V) columns; a frame of n updates is n launches of one persistent kernel
-// (k_batch_step, sized to fill every SM) whose CTAs take (scene, item) pairs from a
-// device-side atomic counter, plus one kernel that advances each scene's step counter.
-// The whole frame is recorded once as a CUDA graph and replayed; the scene table, the
-// work counts and the per-scene time and buffer parity live in device memory, so
-// admitting or removing scenes changes data, not the graph.
+// Single updates: every active scene is cut into work items (BT_ROWS rows x 64 threads x 4
+// columns in FP32, hdr->rows64 x ST_COLS in FP64); a frame of n updates is n launches of one
+// persistent kernel (k_batch_step32, k_batch_step64, sized to fill every SM) whose blocks or
+// warps take items from a device-side atomic counter, plus one kernel that advances each
+// scene's step counter.  The whole frame is recorded once as a CUDA graph and replayed; the
+// scene table, the work counts and the per-scene time and buffer parity live in device
+// memory, so admitting or removing scenes changes data, not the graph.
 //
-// The per-cell arithmetic is the single-scene kernels' (k_step_bulk / fast_edge), so a
+// The per-cell arithmetic is the single-scene kernels' (k_step_bulk, strip64, fast_edge_v), so a
 // scene advanced in a batch is bit-identical to the same scene advanced alone.  FP64
 // scenes update in place (the new level overwrites psi); FP32 scenes (phi and the
 // velocity) write each update into their other pair of fields.
@@ -31,22 +31,20 @@
 #include "wg_scene.h"
 #include "wg_cells.cuh"
 #include "wg_batch.h"
+#include "wg_step64.cuh"
 
 namespace wg {
 
-// A boundary-line cell (reference rules) plus the point source; out of line so that
+// An FP32 boundary-line cell (reference rules) plus the point source; out of line so that
 // the tile loop below stays small.  Its arguments are plain pointers and values: the
 // rule's argument block is built here, in registers of this call, not passed by address
 // (an address taken across the call would put the block in local memory).
-// FP64 fields: phi and psi (y = the cell's psi); returns the new value.
-// FP32 fields: phi and the velocity vel; returns the new phi and velocity.
-template <class T>
-__device__ __forceinline__ FastArgs<T> batch_args(const float *cf, const T *phi, const T *psi, const uint32_t *act,
-                                                  const uint32_t *nz)
+__device__ __noinline__ XV batch_edge_v(const DevParams &p, const float *cf, const float *phi, const float *vel,
+                                        const uint32_t *act, const uint32_t *nz, int i, int j, long long time)
 {
-    FastArgs<T> a;
+    FastArgs<float> a;
     a.phi = phi;
-    a.psi = psi;
+    a.psi = vel;
     a.out = nullptr;
     a.vout = nullptr;
     a.act = act;
@@ -66,67 +64,27 @@ __device__ __forceinline__ FastArgs<T> batch_args(const float *cf, const T *phi,
     a.vmaxf = cf[CF_VMAX];
     a.has_ghosts = 0;
     a.do_source = 1;
-    return a;
-}
-__device__ __noinline__ double batch_edge(const DevParams &p, const float *cf, const double *phi, const double *psi,
-                                          const uint32_t *act, const uint32_t *nz, int i, int j, long long time,
-                                          double y)
-{
-    const FastArgs<double> a = batch_args<double>(cf, phi, psi, act, nz);
-    double v = fast_edge<double, WG_COEF_MASK>(p, a, i, j, time, y);
-    if (p.src_on && i == p.src_i && j == p.src_j) v = A_(v, point_source(p, time));
-    return v;
-}
-__device__ __noinline__ XV batch_edge_v(const DevParams &p, const float *cf, const float *phi, const float *vel,
-                                        const uint32_t *act, const uint32_t *nz, int i, int j, long long time)
-{
-    const FastArgs<float> a = batch_args<float>(cf, phi, vel, act, nz);
     XV r = fast_edge_v<WG_COEF_MASK>(p, a, i, j, time);
     if (p.src_on && i == p.src_i && j == p.src_j) r = source32(r, point_source(p, time));
     return r;
 }
 
 // The scene values the bulk update reads, held in registers for a work item (the
-// descriptor lives in global memory, which the tile's stores could alias); the
-// coefficients in the field precision only.
-template <class T>
+// descriptor lives in global memory, which the tile's stores could alias).
 struct TileCoef {
     int nx, ny, pitch, wpitch, twospeeds, floor_clamp;
-    T c2, c2b, gam, gamb, kappa;
+    float c2, c2b, gam, gamb, kappa;
 };
 
-// One work item.  FP64 (in place): phi, and psi = out, overwritten by the new level.
-// FP32: phi and the velocity vin; the new phi and velocity go to out and vout.
-// Z (FP64 scenes): upd64's flags for KAPPA = 0 and GAMMA = GAMMAB = 0, the bulk update
-// without those zero terms (values unchanged).
-template <class T, int Z = 0>
-__device__ __forceinline__ void batch_tile(const DevParams &p, const float *cf, const T *__restrict__ phi,
-                                           const T *__restrict__ vin, T *__restrict__ out, T *__restrict__ vout,
-                                           const uint32_t *__restrict__ act, const uint32_t *__restrict__ nz, int i0,
-                                           int jt, long long time)
+// One FP32 work item: phi and the velocity vin; the new phi and velocity go to out and vout.
+__device__ __forceinline__ void batch_tile(const DevParams &p, const float *cf, const float *__restrict__ phi,
+                                           const float *__restrict__ vin, float *__restrict__ out,
+                                           float *__restrict__ vout, const uint32_t *__restrict__ act,
+                                           const uint32_t *__restrict__ nz, int i0, int jt, long long time)
 {
-    constexpr int V = Vec<T>::n;
-    constexpr bool F32 = sizeof(T) == 4;
-    TileCoef<T> k;
-    k.nx = p.nx;
-    k.ny = p.ny;
-    k.pitch = p.pitch;
-    k.wpitch = p.wpitch;
-    k.twospeeds = p.twospeeds;
-    k.floor_clamp = p.floor_clamp;
-    if constexpr (F32) {
-        k.c2 = cf[CF_C2];
-        k.c2b = cf[CF_C2B];
-        k.gam = cf[CF_GAM];
-        k.gamb = cf[CF_GAMB];
-        k.kappa = cf[CF_KAPPA];
-    } else {
-        k.c2 = p.c2;
-        k.c2b = p.c2b;
-        k.gam = p.gam;
-        k.gamb = p.gamb;
-        k.kappa = p.kappa;
-    }
+    constexpr int V = Vec<float>::n;
+    const TileCoef k{p.nx, p.ny, p.pitch, p.wpitch, p.twospeeds, p.floor_clamp,
+                     cf[CF_C2], cf[CF_C2B], cf[CF_GAM], cf[CF_GAMB], cf[CF_KAPPA]};
     const float vmaxf = cf[CF_VMAX];
     const int j0 = (jt * BT_THREADS + (int)threadIdx.x) * V;
     // interior rows: the bulk rule (boundary columns and padding take the unwritten-cell
@@ -135,57 +93,43 @@ __device__ __forceinline__ void batch_tile(const DevParams &p, const float *cf, 
         const int i = i0 + rr;
         if (i >= k.nx - 1 || i == 0 || j0 >= k.pitch) continue;
         const size_t row = (size_t)i * k.pitch;
-        T c[V], y[V], n[V], s[V];
+        float c[V], y[V], n[V], s[V];
         vload(phi + row + j0, c);
         vload(vin + row + j0, y);
         vload(phi + row + k.pitch + j0, n);
         vload(phi + row - k.pitch + j0, s);
-        const T wl = (j0 > 0) ? phi[row + j0 - 1] : (T)0;
-        const T er = (j0 + V < k.pitch) ? phi[row + j0 + V] : (T)0;
+        const float wl = (j0 > 0) ? phi[row + j0 - 1] : 0.f;
+        const float er = (j0 + V < k.pitch) ? phi[row + j0 + V] : 0.f;
         const uint32_t word = act[(size_t)i * k.wpitch + (j0 >> 5)] >> (j0 & 31);
-        T o[V], ov[V];
+        float o[V], ov[V];
 #pragma unroll
         for (int q = 0; q < V; q++) {
             const int j = j0 + q;
             const bool ac = (word >> q) & 1u;
             const bool upd = j >= 1 && j < k.ny - 1 && (k.twospeeds || ac);
-            const T x = c[q];
-            const T w = (q == 0) ? wl : c[q - 1];
-            const T e = (q == V - 1) ? er : c[q + 1];
-            if constexpr (!F32) {
-                double v = y[q];
-                if (upd) {
-                    const double delta = L4_(A_(A_(A_(n[q], s[q]), e), w), x);
-                    v = upd64<Z>(x, y[q], ac ? k.c2 : k.c2b, delta, k.kappa, ac ? k.gam : k.gamb);
-                    if (k.floor_clamp && ac) v = floor_clamp(p, v);
-                }
-                o[q] = (T)v;
-            } else {
-                XV r = keep32(x, y[q]);
-                if (upd) {
-                    const float delta = ((n[q] - x) + (s[q] - x)) + ((e - x) + (w - x));
-                    r = upd32(x, y[q], ac ? k.c2 : k.c2b, delta, k.kappa, ac ? k.gam : k.gamb);
-                    if (k.floor_clamp && ac) r = clamp32(x, r, vmaxf);
-                }
-                o[q] = r.x;
-                ov[q] = r.v;
+            const float x = c[q];
+            const float w = (q == 0) ? wl : c[q - 1];
+            const float e = (q == V - 1) ? er : c[q + 1];
+            XV r = keep32(x, y[q]);
+            if (upd) {
+                const float delta = ((n[q] - x) + (s[q] - x)) + ((e - x) + (w - x));
+                r = upd32(x, y[q], ac ? k.c2 : k.c2b, delta, k.kappa, ac ? k.gam : k.gamb);
+                if (k.floor_clamp && ac) r = clamp32(x, r, vmaxf);
             }
+            o[q] = r.x;
+            ov[q] = r.v;
         }
         vstore(out + row + j0, o);
-        if constexpr (F32) vstore(vout + row + j0, ov);
+        vstore(vout + row + j0, ov);
     }
     // then the boundary lines and the point source, by the threads that stored those
-    // cells above (each reads phi and its own cell's psi or velocity)
+    // cells above (each reads phi and its own cell's velocity)
     const bool col0 = j0 == 0, colr = k.ny - 1 >= j0 && k.ny - 1 < j0 + V;
     const bool srcj = p.src_on && p.src_j >= j0 && p.src_j < j0 + V && p.src_j > 0 && p.src_j < k.ny - 1;
     auto edge = [&](size_t row, int i, int j) {
-        if constexpr (F32) {
-            const XV r = batch_edge_v(p, cf, phi, vin, act, nz, i, j, time);
-            out[row + j] = r.x;
-            vout[row + j] = r.v;
-        } else {
-            out[row + j] = batch_edge(p, cf, phi, out, act, nz, i, j, time, out[row + j]);
-        }
+        const XV r = batch_edge_v(p, cf, phi, vin, act, nz, i, j, time);
+        out[row + j] = r.x;
+        vout[row + j] = r.v;
     };
     for (int rr = threadIdx.y; rr < BT_ROWS; rr += blockDim.y) {
         const int i = i0 + rr;
@@ -203,21 +147,20 @@ __device__ __forceinline__ void batch_tile(const DevParams &p, const float *cf, 
         if (colr) edge(row, i, k.ny - 1);
         if (srcj && i == p.src_i) {
             const double add = point_source(p, time);
-            out[row + p.src_j] = (T)A_((double)out[row + p.src_j], add);
-            if constexpr (F32) vout[row + p.src_j] = (T)A_((double)vout[row + p.src_j], add);
+            out[row + p.src_j] = (float)A_((double)out[row + p.src_j], add);
+            vout[row + p.src_j] = (float)A_((double)vout[row + p.src_j], add);
         }
     }
 }
 
-// Persistent blocks take work items (BT_ROWS rows x one column tile of one scene) from
+// Persistent blocks take FP32 work items (BT_ROWS rows x one column tile of one scene) from
 // a device counter.  Each item's scene entry, first row, column tile and slot come from
 // one int4 of the item table built with the scene table.  The ticket of the following
 // item is taken while this one runs, and read after it, so its latency is hidden.
 // all = 0: only the items of scenes without skewed passes (the first plain_tiles).
-template <class T>
-__global__ void __launch_bounds__(256, 4) k_batch_step(const BatchHdr *__restrict__ hdr, const SlotDev *__restrict__ tab,
-                                                    const int4 *__restrict__ items, SlotDyn *__restrict__ dyn,
-                                                    int *__restrict__ counter, int u, int all)
+__global__ void __launch_bounds__(256, 4) k_batch_step32(const BatchHdr *__restrict__ hdr, const SlotDev *__restrict__ tab,
+                                                         const int4 *__restrict__ items, SlotDyn *__restrict__ dyn,
+                                                         int *__restrict__ counter, int u, int all)
 {
     __shared__ int s_next[2];
     pdl_wait();  // launched by launch_pdl: the previous update has completed
@@ -234,32 +177,57 @@ __global__ void __launch_bounds__(256, 4) k_batch_step(const BatchHdr *__restric
         const int4 w = items[it];
         const SlotDev &sd = tab[w.x];
         const SlotDyn d = dyn[w.w];
-        const T *in, *vin;
-        T *out, *vout;
-        if constexpr (sizeof(T) == 4) {  // pair (pair ^ u) -> the other pair
-            const int pin = d.pair ^ (u & 1);
-            in = (const T *)sd.f[2 * pin];
-            vin = (const T *)sd.f[2 * pin + 1];
-            out = (T *)sd.f[2 * (pin ^ 1)];
-            vout = (T *)sd.f[2 * (pin ^ 1) + 1];
-        } else {  // in place within pair 0
-            const int phase = (d.cur + u) & 1;
-            in = (const T *)sd.f[phase];
-            out = (T *)sd.f[1 - phase];
-            vin = out;
-            vout = nullptr;
-        }
-        int z = 0;  // block-uniform
-        if constexpr (sizeof(T) == 8)
-            z = (sd.p.kappa == 0.0 ? Z_KAPPA : 0) | (sd.p.gam == 0.0 && sd.p.gamb == 0.0 ? Z_GAMMA : 0);
-        if (z == (Z_KAPPA | Z_GAMMA))
-            batch_tile<T, Z_KAPPA | Z_GAMMA>(sd.p, sd.cf, in, vin, out, vout, sd.act, sd.nz, w.y, w.z, d.time + u + 1);
-        else if (z == Z_KAPPA)
-            batch_tile<T, Z_KAPPA>(sd.p, sd.cf, in, vin, out, vout, sd.act, sd.nz, w.y, w.z, d.time + u + 1);
-        else
-            batch_tile<T>(sd.p, sd.cf, in, vin, out, vout, sd.act, sd.nz, w.y, w.z, d.time + u + 1);
+        const int pin = d.pair ^ (u & 1);  // pair (pair ^ u) -> the other pair
+        batch_tile(sd.p, sd.cf, (const float *)sd.f[2 * pin], (const float *)sd.f[2 * pin + 1], (float *)sd.f[2 * (pin ^ 1)],
+                   (float *)sd.f[2 * (pin ^ 1) + 1], sd.act, sd.nz, w.y, w.z, d.time + u + 1);
         if (tid == 0) s_next[buf ^ 1] = next;
         __syncthreads();  // the next ticket is visible; s_next[buf] is free again
+    }
+}
+
+// FP64 items: strips of hdr->rows64 rows x ST_COLS columns (wg_step64.cuh), or 32 cells of the
+// boundary lines (first row 0), one warp and one ticket each, in place within pair 0.  The scene's parameters are staged in the warp's shared
+// memory.
+__global__ void __launch_bounds__(128, 4) k_batch_step64(const BatchHdr *__restrict__ hdr, const SlotDev *__restrict__ tab,
+                                                         const int4 *__restrict__ items, SlotDyn *__restrict__ dyn,
+                                                         int *__restrict__ counter, int u, int all)
+{
+    __shared__ DevParams s_p[4];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    DevParams &p = s_p[wid];
+    pdl_wait();  // launched by launch_pdl: the previous update has completed
+    pdl_trigger();
+    const int total = all ? hdr->total_tiles : hdr->plain_tiles;
+    int next = 0;
+    if (lane == 0) next = atomicAdd(counter + u, 1);
+    for (;;) {
+        const int it = __shfl_sync(0xffffffffu, next, 0);
+        if (it >= total) break;  // warp-uniform
+        if (lane == 0) next = atomicAdd(counter + u, 1);  // read after this item: its latency is hidden
+        const int4 w = items[it];
+        const SlotDev &sd = tab[w.x];
+        __syncwarp();  // every lane is done with the previous item's parameters
+        {
+            const int *src = reinterpret_cast<const int *>(&sd.p);
+            int *dst = reinterpret_cast<int *>(&p);
+            for (int k = lane; k < (int)(sizeof(DevParams) / 4); k += 32) dst[k] = src[k];
+        }
+        __syncwarp();
+        const SlotDyn d = dyn[w.w];
+        const int phase = (d.cur + u) & 1;
+        const Strip64 a{(const double *)sd.f[phase], (const double *)sd.f[1 - phase], (double *)sd.f[1 - phase], sd.act, sd.nz,
+                        nullptr, nullptr, nullptr, nullptr, 0, 1};
+        const int r1 = min(w.y + hdr->rows64, p.nx - 1);
+        const long long t = d.time + u + 1;
+        if (w.y == 0) {  // 32 boundary-line cells
+            const int q = w.z * 32 + lane;
+            if (q < edge64_cells(p)) edge64_cell<WG_COEF_MASK, false>(p, a, q, t);
+            continue;
+        }
+        const int z = (p.kappa == 0.0 ? Z_KAPPA : 0) | (p.gam == 0.0 && p.gamb == 0.0 ? Z_GAMMA : 0);
+        if (z == (Z_KAPPA | Z_GAMMA)) strip64<WG_COEF_MASK, false, Z_KAPPA | Z_GAMMA>(p, a, w.z * ST_COLS, w.y, r1, t);
+        else if (z == Z_KAPPA) strip64<WG_COEF_MASK, false, Z_KAPPA>(p, a, w.z * ST_COLS, w.y, r1, t);
+        else strip64<WG_COEF_MASK, false, 0>(p, a, w.z * ST_COLS, w.y, r1, t);
     }
 }
 
@@ -456,14 +424,22 @@ static wg_status build_list(wg_batch *b, int K, int d, const std::vector<int> &t
 
 wg_status batch_refresh_table(wg_batch *b)
 {
-    constexpr int Vf = 4, Vd = 2;
-    const int V = (b->prec == WG_FP32) ? Vf : Vd;
+    constexpr int V = Vec<float>::n;
     std::vector<SlotDev> tab;
     std::vector<int> tab_slot;
     std::vector<int4> items;
     int base = 0, plain = 0, nskew = 0, nwrap = 0;
     long long cells = 0;
     unsigned sig = 0;
+    // FP64: rows of a strip, about three items per resident warp
+    int rows64 = BT_ROWS;
+    if (b->prec == WG_FP64) {
+        long long strip_rows = 0;
+        for (const BatchSlotHost &h : b->slots)
+            if (h.used) strip_rows += (long long)(h.prm.nx - 2) * ((h.prm.ny + ST_COLS - 1) / ST_COLS);
+        const long long warps = 4LL * b->persistent_blocks;
+        rows64 = (int)std::min(64LL, std::max(2LL, (strip_rows + 3 * warps - 1) / (3 * warps)));
+    }
     // scenes without skewed passes first: their items are the first plain_tiles
     for (int pass = 0; pass < 2; pass++) {
         for (int k = 0; k < (int)b->slots.size(); k++) {
@@ -486,13 +462,18 @@ wg_status batch_refresh_table(wg_batch *b)
             }
             d.skew_k = sk;
             d.wrap = h.wrap ? 1 : 0;
-            d.tiles_j = (h.dp.pitch / V + BT_THREADS - 1) / BT_THREADS;
-            const int tiles_i = (h.prm.nx + BT_ROWS - 1) / BT_ROWS;
-            d.ntiles = tiles_i * d.tiles_j;
+            // FP64: the boundary lines (row 0 as the mark of such an item), then strips of the interior
+            const bool f64 = b->prec == WG_FP64;
+            d.tiles_j = f64 ? (h.prm.ny + ST_COLS - 1) / ST_COLS : (h.dp.pitch / V + BT_THREADS - 1) / BT_THREADS;
+            const int first = f64 ? 1 : 0, step = f64 ? rows64 : BT_ROWS, tiles_i = (h.prm.nx - 2 * first + step - 1) / step;
+            const int edges = f64 ? (edge64_cells(h.dp) + 31) / 32 : 0;
+            d.ntiles = edges + tiles_i * d.tiles_j;
             d.tile_base = base;
             base += d.ntiles;
+            for (int q = 0; q < edges; q++) items.push_back(make_int4((int)tab.size(), 0, q, k));
             for (int ti = 0; ti < tiles_i; ti++)
-                for (int tj = 0; tj < d.tiles_j; tj++) items.push_back(make_int4((int)tab.size(), ti * BT_ROWS, tj, k));
+                for (int tj = 0; tj < d.tiles_j; tj++)
+                    items.push_back(make_int4((int)tab.size(), first + ti * step, tj, k));
             cells += (long long)h.prm.nx * h.prm.ny;
             if (sk > 0) {
                 sig |= 1u << sk;
@@ -531,7 +512,7 @@ wg_status batch_refresh_table(wg_batch *b)
         WG_CUDA(cudaMemcpyAsync(b->d_tab, tab.data(), sizeof(SlotDev) * tab.size(), cudaMemcpyHostToDevice, b->st));
         WG_CUDA(cudaMemcpyAsync(b->d_items, items.data(), sizeof(int4) * items.size(), cudaMemcpyHostToDevice, b->st));
     }
-    BatchHdr h{(int)tab.size(), base, plain, 0};
+    BatchHdr h{(int)tab.size(), base, plain, rows64};
     WG_CUDA(cudaMemcpyAsync(b->d_hdr, &h, sizeof h, cudaMemcpyHostToDevice, b->st));
     WG_CUDA(cudaStreamSynchronize(b->st));
     b->nactive = (int)tab.size();
@@ -635,9 +616,10 @@ static void batch_enqueue_frame(wg_batch *b, int n, bool skewed)
         }
     }
     if (!skewed || (b->graph_sig & 1u)) {  // the chain of single updates
-        dim3 blk(BT_THREADS, 4);
+        const bool f32 = sizeof(T) == 4;
         for (int u = 0; u < n; u++)
-            launch_pdl(k_batch_step<T>, dim3(b->persistent_blocks), blk, 0, b->st, (const BatchHdr *)b->d_hdr,
+            launch_pdl(f32 ? k_batch_step32 : k_batch_step64, dim3(b->persistent_blocks),
+                       f32 ? dim3(BT_THREADS, 4) : dim3(128), 0, b->st, (const BatchHdr *)b->d_hdr,
                        (const SlotDev *)b->d_tab, (const int4 *)b->d_items, b->d_dyn, b->d_counter, u, skewed ? 0 : 1);
     }
     for (int K : groups) cudaStreamWaitEvent(b->st, b->ev_join[K], 0);
@@ -802,8 +784,8 @@ wg_status wg_batch_create(int32_t precision, void *stream, wg_batch **out)
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
         e = (precision == WG_FP32)
-                ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<float>, BT_THREADS * 4, 0)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step<double>, BT_THREADS * 4, 0);
+                ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step32, BT_THREADS * 4, 0)
+                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batch_step64, 128, 0);
     if (e == cudaSuccess) e = cudaHostAlloc(&b->h_out, 16 * sizeof(double), cudaHostAllocDefault);
     b->skew_n_cap = 32;
     if (e == cudaSuccess) e = cudaMalloc(&b->d_skew_n, sizeof(int) * b->skew_n_cap);

@@ -32,7 +32,8 @@ struct SlotDyn {
 };
 struct BatchHdr {
     int nactive, total_tiles;    // all work items
-    int plain_tiles, pad_;       // items of the scenes without skewed passes (they come first)
+    int plain_tiles;             // items of the scenes without skewed passes (they come first)
+    int rows64;                  // rows of an FP64 item
 };
 
 constexpr int BATCH_CLASSES = 16;   // size classes: floor(log2(cells)) - 10, clamped to 0..15

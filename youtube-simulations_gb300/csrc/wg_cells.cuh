@@ -129,25 +129,4 @@ __device__ inline XV fast_edge_v(const DevParams &p, const FastArgs<float> &a, i
     return r;
 }
 
-// Boundary-line cell of the native FP64 form, reference rules.  Returns the value to
-// store (the old psi value y when the reference writes nothing).
-template <class T, int COEF>
-__device__ inline T fast_edge(const DevParams &p, const FastArgs<T> &a, int i, int j, long long time, T y)
-{
-    Field<T> PHI{a.phi, p.pitch}, PSI{a.psi, p.pitch};
-    ActBits ACT{a.act, p.wpitch}, NZ{a.nz, p.wpitch};
-    double v;
-    bool w;
-    if (COEF == WG_COEF_MASK) {
-        CoefMask CF{ACT, p.c2, p.c2b, p.gam, p.gamb, p.courant, p.courantb};
-        w = edge_cell<T>(p, time, i, j, PHI, PSI, ACT, CF, &v);
-    } else {
-        CoefTab<T> CF{a.tcc, a.tc, a.tg, p.pitch, p.gam};
-        w = edge_cell<T>(p, time, i, j, PHI, PSI, ACT, CF, &v);
-    }
-    if (!w) v = (double)y;
-    if (p.floor_clamp && NZ(i, j)) v = floor_clamp(p, v);
-    return (T)v;
-}
-
 }  // namespace wg

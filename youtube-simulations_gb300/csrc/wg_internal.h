@@ -77,8 +77,9 @@ void launch_step_exact_energy(const DevParams &p, const double *phi, const doubl
 void launch_neumann_exact(const DevParams &p, const double *phi, double *out, const int16_t *xy,
                           const wg_neumann_bc *rec, int n, cudaStream_t st);
 template <class T> void launch_point_source(const DevParams &p, T *out, T *vout, long long time, cudaStream_t st);
-template <class T> void launch_step_fast(const DevParams &p, const FastArgs<T> &a, int coef_mode, long long time,
-                                         cudaStream_t st);
+// one update; returns the number of kernels launched
+template <class T> int launch_step_fast(const DevParams &p, const FastArgs<T> &a, int coef_mode, long long time,
+                                        cudaStream_t st);
 template <class T> void launch_neumann_fast(const DevParams &p, const T *phi, T *out, T *vout, const int4 *idx,
                                             const double2 *w, int n, cudaStream_t st);
 template <class T> void launch_energy(const DevParams &p, const T *phi, const T *psi, const int16_t *xy,

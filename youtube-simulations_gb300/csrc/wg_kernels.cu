@@ -1,63 +1,70 @@
 // wg_kernels.cu — single-update stepping kernels, Neumann gather, point source,
 // energy reductions and small utility kernels for sm_103a.
 //
-//  k_step_exact   drop-in form: int16 mask, FP64 tables, three buffers, writes exactly
-//                 the cells wave_billiard.c:302-610 writes (bit-identical FP64).
-//  k_step_bulk    native form, interior rows: 1-bit masks, 16-byte vector loads along
-//                 j; FP64 (reference operation order) in place (the new level
-//                 overwrites psi), or FP32 (phi and velocity, increment form) into the
-//                 other pair of fields.
-//  k_step_edge    native form, the four boundary lines and the point source.
+//  k_step64       FP64 update in the reference's operation order, of native scenes (in
+//                 place, the new level overwrites psi) and of the drop-in (int16 mask,
+//                 tables, three buffers, writes exactly the cells wave_billiard.c:302-610
+//                 writes; bit-identical).
+//  k_step_bulk    FP32 update, interior rows: 1-bit masks, 16-byte vector loads along j;
+//                 phi and velocity, increment form, into the other pair of fields.
+//  k_step_edge    FP32, the four boundary lines and the point source.
 //  k_neumann      Neumann gather of wave_billiard.c:379-389 for the active records.
 //  k_energy_cols  compute_energy (wave_common.c:453-472) per cell, one warp per
 //                 column: sums of j < ny/2 and j >= ny/2, box partials per block.
 //  k_energy_final total and the six compute_energy_tblr boxes from the partials.
+#include <algorithm>
 #include <type_traits>
 #include "wg_internal.h"
 #include "wg_cells.cuh"
+#include "wg_step64.cuh"
 
 namespace wg {
 
 // ---------------------------------------------------------------------------
-// Exact drop-in kernel
+// FP64 updates (scenes and the drop-in)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_step_exact(DevParams p, const double *__restrict__ phi,
-                                                    const double *__restrict__ psi, double *__restrict__ out,
-                                                    const int16_t *__restrict__ xy, const double *__restrict__ tcc,
-                                                    const double *__restrict__ tc, const double *__restrict__ tg,
-                                                    long long time, int do_source)
+// One update: blocks of boundary-line cells, then a warp per strip of ST_COLS columns and `rows`
+// rows (wg_step64.cuh).  3840x2160 two-medium table, GAMMA = 1e-4: 104 us an update
+// (80 Gcell/s, FP64 pipe 75% busy), 166 with every operation on the FP64 pipe and the edge lines
+// in a second launch; 1280x720 ellipse, no GAMMA: 10.6 us against 14.2.  16 warps per SM: 128
+// registers (96 spill and measured 12% slower on tables).
+template <int COEF, bool EXACT, int Z>
+__global__ void __launch_bounds__(128, 4) k_step64(const __grid_constant__ DevParams p, const __grid_constant__ Strip64 a,
+                                                   int edge_blocks, int strips, int rows, long long time)
 {
     pdl_wait();  // launched by launch_pdl: the previous update has completed
     pdl_trigger();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= p.nx || j >= p.ny) return;
-    const size_t c = (size_t)i * p.pitch + j;
-    const int m = xy[c];
-    double v = 0.0;
-    bool w;
-    if (i == 0 || i == p.nx - 1 || j == 0 || j == p.ny - 1) {
-        Field<double> PHI{phi, p.pitch}, PSI{psi, p.pitch};
-        ActI16 ACT{xy, p.pitch};
-        CoefTab<double> CF{tcc, tc, tg, p.pitch, 0.0};
-        w = edge_cell<double>(p, time, i, j, PHI, PSI, ACT, CF, &v);
-    } else {
-        w = p.twospeeds || m > 0;
-        if (w) {
-            const double x = phi[c], y = psi[c];
-            const double delta = L4_(A_(A_(A_(phi[c + p.pitch], phi[c - p.pitch]), phi[c + 1]), phi[c - 1]), x);
-            v = upd64(x, y, tcc[c], delta, p.kappa, tg[c]);
-        }
+    if ((int)blockIdx.x < edge_blocks) {  // a thread per boundary-line cell
+        const int q = blockIdx.x * 128 + threadIdx.x;
+        if (q < edge64_cells(p)) edge64_cell<COEF, EXACT>(p, a, q, time);
+        return;
     }
-    if (p.floor_clamp && m != 0) {
-        if (!w) { v = out[c]; w = true; }
-        v = floor_clamp(p, v);
+    const int w = ((int)blockIdx.x - edge_blocks) * 4 + (threadIdx.x >> 5);
+    const int chunk = w / strips, base = (w - chunk * strips) * ST_COLS, r0 = 1 + chunk * rows;
+    if (r0 >= p.nx - 1) return;  // warp-uniform
+    strip64<COEF, EXACT, Z>(p, a, base, r0, min(r0 + rows, p.nx - 1), time);
+}
+
+template <int COEF, bool EXACT, int Z>
+static void launch_step64_z(const DevParams &p, const Strip64 &a, long long time, cudaStream_t st)
+{
+    static int resident = 0;  // warps on the device
+    if (!resident) {
+        int dev = 0, sms = 0, per = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step64<COEF, EXACT, Z>, 128, 0);
+        resident = std::max(1, sms) * std::max(1, per) * 4;
     }
-    if (do_source && p.src_on && i == p.src_i && j == p.src_j) {
-        if (!w) { v = out[c]; w = true; }
-        v = A_(v, point_source(p, time));
-    }
-    if (w) out[c] = v;
+    // about three waves of warps: fewer leave SMs idle behind strips outside the domain, more
+    // unpack too many rows twice (1280x720 ellipse, us an update by rows of a strip: 1: 12.0,
+    // 2: 9.9, 3: 9.6 (chosen), 4: 10.1, 7: 10.9; 1920x1080 table: 3: 20.5, 5: 19.9 (chosen), 8: 20.6)
+    const int strips = (p.ny + ST_COLS - 1) / ST_COLS;
+    const int rows = (int)std::min(256LL, std::max(1LL, ((long long)(p.nx - 2) * strips + 3LL * resident - 1) / (3LL * resident)));
+    const long long warps = (long long)strips * ((p.nx - 2 + rows - 1) / rows);
+    const int edge_blocks = (edge64_cells(p) + 127) / 128;
+    launch_pdl(k_step64<COEF, EXACT, Z>, dim3((unsigned)(edge_blocks + (warps + 3) / 4)), dim3(128), 0, st, p, a, edge_blocks,
+               strips, rows, time);
 }
 
 // wave_energy's stepper (wave_energy.c:662-913) on the half domain j < ny/2, with
@@ -188,81 +195,66 @@ __global__ void k_point_source(DevParams p, T *out, T *vout, long long time)
 // ---------------------------------------------------------------------------
 // Fast native kernel
 // ---------------------------------------------------------------------------
-// Interior rows 1..nx-2 of one update: each thread updates V = 16/sizeof(T) consecutive
-// cells of row i with every load (three phi rows, psi or the velocity, tcc, the j-1 / j+V
-// neighbours, the mask word) issued before the first use.  FP64: in place, the new level
-// overwriting psi.  FP32: the new phi and velocity into the other pair.  Boundary-line
-// cells (j = 0, j = ny-1) and padding take the rule of an unwritten cell; k_step_edge
-// computes the boundary lines afterwards.
-template <class T, int COEF, int Z = 0>
+// Interior rows 1..nx-2 of one FP32 update: each thread updates four consecutive cells of
+// row i with every load (three phi rows, the velocity, tcc, the j-1 / j+4 neighbours, the
+// mask word) issued before the first use, the new phi and velocity into the other pair.
+// Boundary-line cells (j = 0, j = ny-1) and padding take the rule of an unwritten cell;
+// k_step_edge computes the boundary lines afterwards.
+template <int COEF>
 __global__ void __launch_bounds__(256) k_step_bulk(const __grid_constant__ DevParams p,
-                                                   const __grid_constant__ FastArgs<T> a)
+                                                   const __grid_constant__ FastArgs<float> a)
 {
-    constexpr int V = Vec<T>::n;
+    constexpr int V = Vec<float>::n;
     pdl_wait();  // launched by launch_pdl: the previous update has completed
     pdl_trigger();
     const int i = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     const int j0 = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (i >= p.nx - 1 || j0 >= p.pitch) return;
     const size_t row = (size_t)i * p.pitch;
-    T c[V], y[V], n[V], s[V], cc[V];
+    float c[V], y[V], n[V], s[V], cc[V];
     vload(a.phi + row + j0, c);
     vload(a.psi + row + j0, y);
     vload(a.phi + row + p.pitch + j0, n);
     vload(a.phi + row - p.pitch + j0, s);
     if (COEF == WG_COEF_TABLE) vload(a.tcc + row + j0, cc);
-    const T wl = (j0 > 0) ? a.phi[row + j0 - 1] : (T)0;
-    const T er = (j0 + V < p.pitch) ? a.phi[row + j0 + V] : (T)0;
+    const float wl = (j0 > 0) ? a.phi[row + j0 - 1] : 0.f;
+    const float er = (j0 + V < p.pitch) ? a.phi[row + j0 + V] : 0.f;
     const uint32_t word = a.act[(size_t)i * p.wpitch + (j0 >> 5)] >> (j0 & 31);
     uint32_t nzw = 0;
     if (p.floor_clamp && a.has_ghosts) nzw = a.nz[(size_t)i * p.wpitch + (j0 >> 5)] >> (j0 & 31);
-    T out[V], vo[V];
+    float out[V], vo[V];
 #pragma unroll
     for (int k = 0; k < V; k++) {
         const int j = j0 + k;
         const bool act = (word >> k) & 1u;
         const bool upd = j >= 1 && j < p.ny - 1 && (p.twospeeds || act);
         const bool clamp = p.floor_clamp && j >= 1 && j < p.ny - 1 && ((upd && act) || ((nzw >> k) & 1u));
-        const T x = c[k];
-        const T w = (k == 0) ? wl : c[k - 1];
-        const T e = (k == V - 1) ? er : c[k + 1];
-        if constexpr (sizeof(T) == 8) {
-            double v = y[k];
-            if (upd) {
-                const double delta = L4_(A_(A_(A_(n[k], s[k]), e), w), x);
-                const double ccv = (COEF == WG_COEF_TABLE) ? (double)cc[k] : (act ? p.c2 : p.c2b);
-                double g;
-                if (COEF == WG_COEF_TABLE) g = a.tg ? (double)a.tg[row + j] : p.gam;
-                else g = act ? p.gam : p.gamb;
-                v = upd64<Z>(x, y[k], ccv, delta, p.kappa, g);
-            }
-            if (clamp) v = floor_clamp(p, v);
-            out[k] = (T)v;
-        } else {
-            XV r = keep32(x, y[k]);
-            if (upd) {
-                const float delta = ((n[k] - x) + (s[k] - x)) + ((e - x) + (w - x));
-                const float ccv = (COEF == WG_COEF_TABLE) ? cc[k] : (act ? a.c2f : a.c2bf);
-                float g;
-                if (COEF == WG_COEF_TABLE) g = a.tg ? a.tg[row + j] : a.gamf;
-                else g = act ? a.gamf : a.gambf;
-                r = upd32(x, y[k], ccv, delta, a.kappaf, g);
-            }
-            if (clamp) r = clamp32(x, r, a.vmaxf);
-            out[k] = r.x;
-            vo[k] = r.v;
+        const float x = c[k];
+        const float w = (k == 0) ? wl : c[k - 1];
+        const float e = (k == V - 1) ? er : c[k + 1];
+        XV r = keep32(x, y[k]);
+        if (upd) {
+            const float delta = ((n[k] - x) + (s[k] - x)) + ((e - x) + (w - x));
+            const float ccv = (COEF == WG_COEF_TABLE) ? cc[k] : (act ? a.c2f : a.c2bf);
+            float g;
+            if (COEF == WG_COEF_TABLE) g = a.tg ? a.tg[row + j] : a.gamf;
+            else g = act ? a.gamf : a.gambf;
+            r = upd32(x, y[k], ccv, delta, a.kappaf, g);
         }
+        if (clamp) r = clamp32(x, r, a.vmaxf);
+        out[k] = r.x;
+        vo[k] = r.v;
     }
     vstore(a.out + row + j0, out);
-    if constexpr (sizeof(T) == 4) vstore(a.vout + row + j0, vo);
+    vstore(a.vout + row + j0, vo);
 }
 
-// The four boundary lines of one update (one thread per cell, reference rules) and,
+// The four boundary lines of one FP32 update (one thread per cell, reference rules) and,
 // in the last thread, the point source when it lies inside; runs after k_step_bulk
-// (boundary cells read only phi and their own psi or velocity).
-template <class T, int COEF>
+// (boundary cells read only phi and their own velocity).
+template <int COEF>
 __global__ void __launch_bounds__(256) k_step_edge(const __grid_constant__ DevParams p,
-                                                   const __grid_constant__ FastArgs<T> a, long long time)
+                                                   const __grid_constant__ FastArgs<float> a, long long time)
 {
     pdl_wait();  // launched by launch_pdl: the bulk kernel of this update has completed
     pdl_trigger();
@@ -279,23 +271,17 @@ __global__ void __launch_bounds__(256) k_step_edge(const __grid_constant__ DevPa
             p.src_j < NY - 1) {
             const size_t o = (size_t)p.src_i * p.pitch + p.src_j;
             const double add = point_source(p, time);
-            a.out[o] = (T)A_((double)a.out[o], add);
-            if constexpr (sizeof(T) == 4) a.vout[o] = (T)A_((double)a.vout[o], add);
+            a.out[o] = (float)A_((double)a.out[o], add);
+            a.vout[o] = (float)A_((double)a.vout[o], add);
         }
         return;
     }
     const size_t o = (size_t)i * p.pitch + j;
     const bool src = a.do_source && p.src_on && i == p.src_i && j == p.src_j;
-    if constexpr (sizeof(T) == 8) {
-        T v = fast_edge<T, COEF>(p, a, i, j, time, a.psi[o]);
-        if (src) v = (T)A_((double)v, point_source(p, time));
-        a.out[o] = v;
-    } else {
-        XV r = fast_edge_v<COEF>(p, a, i, j, time);
-        if (src) r = source32(r, point_source(p, time));
-        a.out[o] = r.x;
-        a.vout[o] = r.v;
-    }
+    XV r = fast_edge_v<COEF>(p, a, i, j, time);
+    if (src) r = source32(r, point_source(p, time));
+    a.out[o] = r.x;
+    a.vout[o] = r.v;
 }
 
 // Native Neumann gather: active records only, from phi (level t) into the new level
@@ -667,8 +653,9 @@ void launch_step_exact(const DevParams &p, const double *phi, const double *psi,
                        const double *tcc, const double *tc, const double *tg, long long time, int do_source,
                        cudaStream_t st)
 {
-    dim3 blk(64, 4), grd((p.ny + 63) / 64, (p.nx + 3) / 4);
-    launch_pdl(k_step_exact, grd, blk, 0, st, p, phi, psi, out, xy, tcc, tc, tg, time, do_source);
+    const Strip64 a{phi, psi, out, nullptr, nullptr, xy, tcc, tc, tg, 0, do_source};
+    if (p.kappa == 0.0) launch_step64_z<WG_COEF_TABLE, true, Z_KAPPA>(p, a, time, st);
+    else launch_step64_z<WG_COEF_TABLE, true, 0>(p, a, time, st);
 }
 
 void launch_step_exact_energy(const DevParams &p, const double *phi, const double *psi, double *out,
@@ -699,39 +686,44 @@ void launch_point_source(const DevParams &p, T *out, T *vout, long long time, cu
 template void launch_point_source<float>(const DevParams &, float *, float *, long long, cudaStream_t);
 template void launch_point_source<double>(const DevParams &, double *, double *, long long, cudaStream_t);
 
-// FP64: the bulk update without the terms whose coefficient is zero on every cell
-// (upd64's Z flags: KAPPA = 0; GAMMA = 0 as a uniform value); the values are unchanged.
-template <class T, int COEF>
-static void launch_bulk(const DevParams &p, const FastArgs<T> &a, dim3 grd, dim3 blk, cudaStream_t st)
+// The FP64 update without the terms whose coefficient is zero on every cell (upd64's Z flags:
+// KAPPA = 0; GAMMA = 0 as a uniform value); the values are unchanged.
+template <int COEF>
+static void launch_step64(const DevParams &p, const FastArgs<double> &f, long long time, cudaStream_t st)
 {
-    if constexpr (sizeof(T) == 8) {
-        const bool g0 = (COEF == WG_COEF_TABLE) ? (!a.tg && p.gam == 0.0) : (p.gam == 0.0 && p.gamb == 0.0);
-        switch ((p.kappa == 0.0 ? Z_KAPPA : 0) | (g0 ? Z_GAMMA : 0)) {
-        case Z_KAPPA: launch_pdl(k_step_bulk<T, COEF, Z_KAPPA>, grd, blk, 0, st, p, a); return;
-        case Z_GAMMA: launch_pdl(k_step_bulk<T, COEF, Z_GAMMA>, grd, blk, 0, st, p, a); return;
-        case Z_KAPPA | Z_GAMMA: launch_pdl(k_step_bulk<T, COEF, Z_KAPPA | Z_GAMMA>, grd, blk, 0, st, p, a); return;
-        default: break;
-        }
+    const Strip64 a{f.phi, f.psi, f.out, f.act, f.nz, nullptr, f.tcc, f.tc, f.tg, f.has_ghosts, f.do_source};
+    const bool g0 = (COEF == WG_COEF_TABLE) ? (!f.tg && p.gam == 0.0) : (p.gam == 0.0 && p.gamb == 0.0);
+    switch ((p.kappa == 0.0 ? Z_KAPPA : 0) | (g0 ? Z_GAMMA : 0)) {
+    case Z_KAPPA: launch_step64_z<COEF, false, Z_KAPPA>(p, a, time, st); return;
+    case Z_GAMMA: launch_step64_z<COEF, false, Z_GAMMA>(p, a, time, st); return;
+    case Z_KAPPA | Z_GAMMA: launch_step64_z<COEF, false, Z_KAPPA | Z_GAMMA>(p, a, time, st); return;
+    default: launch_step64_z<COEF, false, 0>(p, a, time, st); return;
     }
-    launch_pdl(k_step_bulk<T, COEF>, grd, blk, 0, st, p, a);
 }
 
-template <class T>
-void launch_step_fast(const DevParams &p, const FastArgs<T> &a, int coef_mode, long long time, cudaStream_t st)
+template <>
+int launch_step_fast<double>(const DevParams &p, const FastArgs<double> &a, int coef_mode, long long time, cudaStream_t st)
 {
-    constexpr int V = Vec<T>::n;
+    if (coef_mode == WG_COEF_MASK) launch_step64<WG_COEF_MASK>(p, a, time, st);
+    else launch_step64<WG_COEF_TABLE>(p, a, time, st);
+    return 1;
+}
+
+template <>
+int launch_step_fast<float>(const DevParams &p, const FastArgs<float> &a, int coef_mode, long long time, cudaStream_t st)
+{
+    constexpr int V = Vec<float>::n;
     dim3 blk(64, 4), grd((p.pitch / V + 63) / 64, (p.nx - 2 + 3) / 4);
     const int nedge = 2 * p.nx + 2 * (p.ny - 2) + 1;
     if (coef_mode == WG_COEF_MASK) {
-        launch_bulk<T, WG_COEF_MASK>(p, a, grd, blk, st);
-        launch_pdl(k_step_edge<T, WG_COEF_MASK>, dim3((nedge + 255) / 256), dim3(256), 0, st, p, a, time);
+        launch_pdl(k_step_bulk<WG_COEF_MASK>, grd, blk, 0, st, p, a);
+        launch_pdl(k_step_edge<WG_COEF_MASK>, dim3((nedge + 255) / 256), dim3(256), 0, st, p, a, time);
     } else {
-        launch_bulk<T, WG_COEF_TABLE>(p, a, grd, blk, st);
-        launch_pdl(k_step_edge<T, WG_COEF_TABLE>, dim3((nedge + 255) / 256), dim3(256), 0, st, p, a, time);
+        launch_pdl(k_step_bulk<WG_COEF_TABLE>, grd, blk, 0, st, p, a);
+        launch_pdl(k_step_edge<WG_COEF_TABLE>, dim3((nedge + 255) / 256), dim3(256), 0, st, p, a, time);
     }
+    return 2;
 }
-template void launch_step_fast<float>(const DevParams &, const FastArgs<float> &, int, long long, cudaStream_t);
-template void launch_step_fast<double>(const DevParams &, const FastArgs<double> &, int, long long, cudaStream_t);
 
 template <class T>
 void launch_neumann_fast(const DevParams &p, const T *phi, T *out, T *vout, const int4 *idx, const double2 *w, int n,

@@ -199,15 +199,14 @@ static FastArgs<T> fast_args(wg_scene *s, int do_source)
     return a;
 }
 
-// One update of the single-step form (k_step_bulk + k_step_edge, Neumann gather, source).
+// One update of the single-step form (k_step64, or k_step_bulk + k_step_edge; Neumann gather, source).
 template <class T>
 static wg_status single_update(wg_scene *s)
 {
     s->time++;
     const bool recs = s->nrec > 0;
     FastArgs<T> a = fast_args<T>(s, recs ? 0 : 1);
-    launch_step_fast<T>(s->dp, a, s->coef, s->time, s->st);  // k_step_bulk + k_step_edge
-    s->launches += 2;
+    s->launches += launch_step_fast<T>(s->dp, a, s->coef, s->time, s->st);
     if (recs) {
         launch_neumann_fast<T>(s->dp, a.phi, a.out, a.vout, s->nidx, s->nw, s->nrec, s->st);
         s->launches++;
