@@ -13,6 +13,7 @@
 // palette is the caller's byte table and the faded colour is rounded to bytes.
 #include <cmath>
 #include "wg_internal.h"
+#include "wg_frame.cuh"
 #include "wg_scene.h"
 
 namespace wg {
@@ -32,115 +33,201 @@ __device__ __forceinline__ double ref_argument(double x, double y)
     return alph;
 }
 
-template <class T, int COEF>
-__global__ void k_frame_rgb8(const __grid_constant__ DevParams p, const T *__restrict__ phi,
-                             const T *__restrict__ psi, const uint32_t *__restrict__ nz, const T *__restrict__ tcc,
-                             const uint8_t *__restrict__ lut, wg_frame_params fp, double *__restrict__ acc,
-                             uint8_t *__restrict__ out, int w, int h)
+// The sampled cell as it is stored: phi, psi (FP64 fields) or the velocity (FP32), and its
+// neighbours' phi, clamped at the edges.
+template <class T>
+struct FrameRaw {
+    T x, y, e, w, n, s;
+    int m, j;
+};
+// The same in FP64; psi of FP32 fields is phi - v (exact in FP64).
+struct FrameCell {
+    double x, y, e, w, n, s;
+    int m, j;
+};
+template <class T>
+__device__ __forceinline__ FrameCell frame_cell(const FrameRaw<T> &r)
 {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x, row = blockIdx.y;
-    if (col >= w || row >= h) return;
-    const int i = col * fp.size, j = row * fp.size;
-    const size_t o = ((size_t)row * w + col) * 3, k = (size_t)row * w + col;
-    const int m = (nz[(size_t)i * p.wpitch + (j >> 5)] >> (j & 31)) & 1u;
-    const int plot = fp.plot;
-    const size_t c = (size_t)i * p.pitch + j;
-    const double x = (double)phi[c];
-    // compute_energy / compute_energy_flux neighbours, clamped at the edges
-    double energy = 0.0, vel = 0.0, gx = 0.0, gy = 0.0;
-    if (plot != WG_P_AMPLITUDE) {
-        const int ip = (i + 1 == p.nx) ? p.nx - 1 : i + 1, im = (i == 0) ? 0 : i - 1;
-        const int jp = (j + 1 == p.ny) ? p.ny - 1 : j + 1, jm = (j == 0) ? 0 : j - 1;
-        const double e = (double)phi[(size_t)ip * p.pitch + j], wv = (double)phi[(size_t)im * p.pitch + j];
-        const double n = (double)phi[(size_t)i * p.pitch + jp], sv = (double)phi[(size_t)i * p.pitch + jm];
-        // psi of FP64 fields; FP32 fields hold the velocity: psi = phi - v (exact in FP64)
-        const double y = sizeof(T) == 4 ? S_(x, (double)psi[c]) : (double)psi[c];
-        if (plot == WG_P_ENERGY_FLUX || plot == WG_P_TOTAL_ENERGY_FLUX) {
-            vel = fabs(S_(x, y));
-            gx = S_(e, wv);
-            gy = S_(n, sv);
+    const double x = (double)r.x;
+    return FrameCell{x, sizeof(T) == 4 ? S_(x, (double)r.y) : (double)r.y, (double)r.e, (double)r.w, (double)r.n, (double)r.s, r.m, r.j};
+}
+
+// wave_value (wave_common.c:1053-1162) without the running sums: q is the mode's updated sum.
+__device__ double frame_value(const DevParams &p, const wg_frame_params &fp, const FrameCell &c, double q)
+{
+    double energy;
+    switch (fp.plot) {
+    case WG_P_AMPLITUDE: return A_(fp.vshift, M_(fp.vscale, c.x));
+    case WG_P_ENERGY: return cell_energy(p, c.x, c.y, c.e, c.w, c.n, c.s, c.m);
+    case WG_P_MIXED: return (c.j > p.ny / 2) ? c.x : cell_energy(p, c.x, c.y, c.e, c.w, c.n, c.s, c.m);
+    case WG_P_MEAN_ENERGY: return D_(q, (double)(fp.time + 1));
+    case WG_P_LOG_ENERGY:
+        energy = cell_energy(p, c.x, c.y, c.e, c.w, c.n, c.s, c.m);
+        if (energy < 1.0e-20) energy = 1.0e-20;
+        return A_(fp.log_shift, M_(fp.log_scale, log(energy)));
+    case WG_P_LOG_MEAN_ENERGY: return A_(fp.log_shift, M_(fp.log_scale, log(D_(q, (double)(fp.time + 1)))));
+    case WG_P_ENERGY_FLUX: {
+        const double vel = fabs(S_(c.x, c.y)), gx = S_(c.e, c.w), gy = S_(c.n, c.s);
+        const double mod = (c.m || p.twospeeds) ? M_(vel, sqrt(A_(M_(gx, gx), M_(gy, gy)))) : 0.0;
+        return M_(mod, fp.flux_scale);
+    }
+    case WG_P_AVERAGE_ENERGY: return q;
+    default:  // WG_P_LOG_AVERAGE_ENERGY
+        return (q == 0.0) ? S_(fp.log_shift, M_(10.0, fp.log_scale)) : A_(fp.log_shift, M_(fp.log_scale, log(q)));
+    }
+}
+
+// The modes drawn by color_scheme_asym_palette.
+__device__ __forceinline__ bool frame_asym(int plot)
+{
+    return plot == WG_P_ENERGY || plot == WG_P_MEAN_ENERGY || plot == WG_P_ENERGY_FLUX || plot == WG_P_AVERAGE_ENERGY;
+}
+
+// The palette index in FP64, as the reference computes it.
+template <class T>
+__device__ __noinline__ int frame_hue64(const DevParams &p, const wg_frame_params &fp, const FrameRaw<T> &c, double q)
+{
+    double amp = M_(fp.color_range, tanh(D_(M_(fp.slope, frame_value(p, fp, frame_cell(c), q)), fp.scale)));
+    if (fp.attenuation != 0.0) amp = M_(amp, exp(-M_((double)fp.time, fp.attenuation)));
+    const double hv = M_(256.0, frame_asym(fp.plot) ? amp : M_(0.5, A_(1.0, amp)));
+    return hv >= 255.0 ? 255 : (hv <= 0.0 ? 0 : (int)hv);
+}
+
+// The index and dimming of WG_P_TOTAL_ENERGY_FLUX, whose sum (mgx, mgy) has been updated.
+__device__ __noinline__ int frame_hue_flux(const wg_frame_params &fp, double mgx, double mgy, double *dim)
+{
+    const double mod = sqrt(A_(M_(mgx, mgx), M_(mgy, mgy)));
+    double arg = ref_argument(mgx, mgy);
+    if (arg < 0.0) arg = A_(arg, 6.283185307);
+    *dim = tanh(M_(mod, fp.flux_scale));
+    double hh = M_(fp.slope, D_(arg, 6.283185307));  // C_ONEDIM_LINEAR with scale 1 (colors_waves.c:198-205)
+    if (hh > 1.0) hh = S_(hh, 1.0);
+    else if (hh < 0.0) hh = A_(hh, 1.0);
+    const double hv = M_(256.0, hh);
+    return hv >= 255.0 ? 255 : (hv <= 0.0 ? 0 : (int)hv);
+}
+
+// value +- err of the modes that need no FP64: LOG_SHIFT + LOG_SCALE*log(q) of q with relative
+// error rel and absolute error tiny
+__device__ __forceinline__ float log_fast(const FrameFast &f, float q, float rel, float tiny, float *err)
+{
+    const float l = logf(q);
+    *err = fabsf(f.log_scale) * (rel + tiny / q + 5e-7f * fabsf(l) + 2e-7f) + 3e-7f * (fabsf(f.log_shift) + fabsf(f.log_scale * l));
+    return f.log_shift + f.log_scale * l;
+}
+
+// One block per tile of pixels, a thread per pixel.  The running sums (acc) are kept column by
+// column (k = col*h + row), as they are read.
+template <class T, int COEF>
+__global__ void __launch_bounds__(FT_ROWS *FT_COLS) k_frame_rgb8(const __grid_constant__ DevParams p, const T *__restrict__ phi,
+                                                       const T *__restrict__ psi, const uint32_t *__restrict__ nz,
+                                                       const T *__restrict__ tcc, const uint8_t *__restrict__ lut,
+                                                       const __grid_constant__ wg_frame_params fp,
+                                                       const __grid_constant__ FrameFast ff, double *__restrict__ acc,
+                                                       uint8_t *__restrict__ out, int w, int h)
+{
+    __shared__ FrameTile sh;
+    const int row = blockIdx.y * FT_ROWS + threadIdx.x, col = blockIdx.x * FT_COLS + threadIdx.y;
+    if (col < w && row < h) {
+        const int i = col * fp.size, j = row * fp.size, plot = fp.plot;
+        uint8_t *o = &sh.c[threadIdx.x][3 * threadIdx.y];
+        const size_t k = (size_t)col * h + row, c = (size_t)i * p.pitch + j;
+        const int m = (nz[(size_t)i * p.wpitch + (j >> 5)] >> (j & 31)) & 1u;
+        const bool drawn = p.twospeeds || m;
+        constexpr bool F32 = sizeof(T) == 4;
+        const T tx = phi[c];
+        FrameRaw<T> raw{tx, (T)0, (T)0, (T)0, (T)0, (T)0, m, j};
+        float value = 0.f, err = INFINITY;  // in FP32, when the mode allows
+        double q = 0.0, dim = 1.0;
+        int hue = -1;
+        if (plot == WG_P_AMPLITUDE) {
+            value = amplitude_fast(ff, (float)tx, &err);
         } else {
-            energy = cell_energy(p, x, y, e, wv, n, sv, m);
+            const int ip = (i + 1 == p.nx) ? p.nx - 1 : i + 1, im = (i == 0) ? 0 : i - 1;
+            const int jp = (j + 1 == p.ny) ? p.ny - 1 : j + 1, jm = (j == 0) ? 0 : j - 1;
+            const T te = phi[(size_t)ip * p.pitch + j], tw = phi[(size_t)im * p.pitch + j];
+            const T tn = phi[(size_t)i * p.pitch + jp], ts = phi[(size_t)i * p.pitch + jm], ty = psi[c];
+            raw = FrameRaw<T>{tx, ty, te, tw, tn, ts, m, j};
+            // the velocity and the differences, rounded once to FP32; the energy from them, all of
+            // its terms of one sign: 12 roundings.  tiny: psi = phi - v loses what lies below 2^-53 of
+            // phi, and squares what lies below the smallest float
+            const auto dif = [](T a, T b) { return F32 ? (float)a - (float)b : (float)S_((double)a, (double)b); };
+            const float x = (float)tx, v = F32 ? (float)ty : dif(tx, ty);
+            const float de = dif(te, tx), dw = dif(tx, tw), dn = dif(tn, tx), ds = dif(tx, ts);
+            const float half = m ? ff.half : ff.halfb, es2 = ff.es2;
+            const float rel = 1.5e-6f, tiny = es2 * (4.5e-16f * fabsf(x) * fabsf(v) + 5e-32f * x * x + 1e-40f);
+            const float en = drawn ? es2 * (v * v + half * ((de * de + dw * dw) + (dn * dn + ds * ds))) : 0.f;
+            switch (plot) {
+            case WG_P_MIXED:
+                if (j > p.ny / 2) {
+                    value = x;
+                    err = 2e-7f * fabsf(x);
+                    break;
+                }  // else the energy
+            case WG_P_ENERGY:
+                value = en;
+                err = rel * en + tiny;
+                break;
+            case WG_P_LOG_ENERGY:
+                value = log_fast(ff, fmaxf(en, 1.0e-20f), rel, tiny, &err);
+                break;
+            case WG_P_ENERGY_FLUX: {
+                const float gx = dif(te, tw), gy = dif(tn, ts), g = sqrtf(gx * gx + gy * gy);
+                value = drawn ? fabsf(v) * g * ff.flux : 0.f;
+                err = rel * fabsf(value) + fabsf(ff.flux) * (g * 4.5e-16f * fabsf(x) + fabsf(v) * 2e-19f) + 1e-37f;
+                break;
+            }
+            case WG_P_TOTAL_ENERGY_FLUX: {
+                const FrameCell fc = frame_cell(raw);
+                const double vel = fabs(S_(fc.x, fc.y));
+                const double fx = drawn ? M_(vel, S_(fc.e, fc.w)) : 0.0, fy = drawn ? M_(vel, S_(fc.n, fc.s)) : 0.0;
+                const double mgx = A_(M_(acc[2 * k], 0.99), fx), mgy = A_(M_(acc[2 * k + 1], 0.99), fy);
+                acc[2 * k] = mgx;
+                acc[2 * k + 1] = mgy;
+                if (drawn) hue = frame_hue_flux(fp, mgx, mgy, &dim);
+                break;
+            }
+            default: {  // the modes with a running sum of the energy, kept in FP64
+                const FrameCell fc = frame_cell(raw);
+                double energy = cell_energy(p, fc.x, fc.y, fc.e, fc.w, fc.n, fc.s, m);
+                if (plot == WG_P_AVERAGE_ENERGY || plot == WG_P_LOG_AVERAGE_ENERGY) {
+                    q = A_(M_(fp.avrg_e_factor, acc[k]), M_(S_(1.0, fp.avrg_e_factor), energy));
+                } else {
+                    if (plot == WG_P_LOG_MEAN_ENERGY && energy == 0.0) energy = 1.0e-20;
+                    q = A_(acc[k], energy);
+                }
+                acc[k] = q;
+                const float qf = (float)q;
+                if (plot == WG_P_MEAN_ENERGY || plot == WG_P_AVERAGE_ENERGY) {
+                    value = plot == WG_P_MEAN_ENERGY ? qf * ff.inv_t : qf;
+                    err = 4e-7f * fabsf(value) + 1e-37f;
+                } else if (qf > 1e-30f) {
+                    value = log_fast(ff, plot == WG_P_LOG_MEAN_ENERGY ? qf * ff.inv_t : qf, 4e-7f, 0.f, &err);
+                }
+                break;
+            }
+            }
+        }
+        if (!drawn) {
+            o[0] = o[1] = o[2] = 0;
+        } else {
+            if (hue < 0 && err < 1e30f) hue = hue_fast(ff, value, err, frame_asym(plot));
+            if (hue < 0) hue = frame_hue64<T>(p, fp, raw, q);
+            if (ff.plain && plot != WG_P_TOTAL_ENERGY_FLUX) {
+#pragma unroll
+                for (int a = 0; a < 3; a++) o[a] = lut[hue * 3 + a];
+            } else {
+                double cc = p.c2;
+                if (fp.fade_in_obstacle) cc = (COEF == WG_COEF_TABLE) ? (double)tcc[c] : (m ? p.c2 : p.c2b);
+                // powf is within 4 ulp, its argument within 3e-7 (a tenth of which counts)
+                float ff32 = (float)dim * (fp.fade ? ff.fade : 1.f);
+                if (fp.fade_in_obstacle) ff32 *= powf((COEF == WG_COEF_TABLE) ? (float)tcc[c] * ff.inv_c2 : (m ? 1.f : ff.ratio_b), 0.1f);
+                if (!colour_fast(lut, hue, ff32, 8e-7f, o)) frame_colour64(fp, lut, hue, dim, cc, p.c2, o);
+            }
         }
     }
-    double value = 0.0, dim = 1.0;
-    int asym = 0, linear = 0;
-    switch (plot) {
-    case WG_P_AMPLITUDE: value = A_(fp.vshift, M_(fp.vscale, x)); break;
-    case WG_P_ENERGY: value = energy; asym = 1; break;
-    case WG_P_MIXED: value = (j > p.ny / 2) ? x : energy; break;
-    case WG_P_MEAN_ENERGY:
-        acc[k] = A_(acc[k], energy);
-        value = D_(acc[k], (double)(fp.time + 1));
-        asym = 1;
-        break;
-    case WG_P_LOG_ENERGY:
-        if (energy < 1.0e-20) energy = 1.0e-20;
-        value = A_(fp.log_shift, M_(fp.log_scale, log(energy)));
-        break;
-    case WG_P_LOG_MEAN_ENERGY:
-        if (energy == 0.0) energy = 1.0e-20;
-        acc[k] = A_(acc[k], energy);
-        value = A_(fp.log_shift, M_(fp.log_scale, log(D_(acc[k], (double)(fp.time + 1)))));
-        break;
-    case WG_P_ENERGY_FLUX: {
-        const double mod = (m || p.twospeeds) ? M_(vel, sqrt(A_(M_(gx, gx), M_(gy, gy)))) : 0.0;
-        value = M_(mod, fp.flux_scale);
-        asym = 1;
-        break;
-    }
-    case WG_P_TOTAL_ENERGY_FLUX: {
-        const double fx = (m || p.twospeeds) ? M_(vel, gx) : 0.0, fy = (m || p.twospeeds) ? M_(vel, gy) : 0.0;
-        const double mgx = A_(M_(acc[2 * k], 0.99), fx), mgy = A_(M_(acc[2 * k + 1], 0.99), fy);
-        acc[2 * k] = mgx;
-        acc[2 * k + 1] = mgy;
-        const double mod = sqrt(A_(M_(mgx, mgx), M_(mgy, mgy)));
-        double arg = ref_argument(mgx, mgy);
-        if (arg < 0.0) arg = A_(arg, 6.283185307);
-        value = D_(arg, 6.283185307);
-        linear = 1;
-        dim = tanh(M_(mod, fp.flux_scale));
-        break;
-    }
-    case WG_P_AVERAGE_ENERGY:
-        acc[k] = A_(M_(fp.avrg_e_factor, acc[k]), M_(S_(1.0, fp.avrg_e_factor), energy));
-        value = acc[k];
-        asym = 1;
-        break;
-    default:  // WG_P_LOG_AVERAGE_ENERGY
-        acc[k] = A_(M_(fp.avrg_e_factor, acc[k]), M_(S_(1.0, fp.avrg_e_factor), energy));
-        value = (acc[k] == 0.0) ? S_(fp.log_shift, M_(10.0, fp.log_scale))
-                                : A_(fp.log_shift, M_(fp.log_scale, log(acc[k])));
-        break;
-    }
-    if (!(p.twospeeds || m)) {
-        out[o] = out[o + 1] = out[o + 2] = 0;
-        return;
-    }
-    double hh;
-    if (linear) {  // C_ONEDIM_LINEAR with scale 1 (colors_waves.c:198-205)
-        hh = M_(fp.slope, value);
-        if (hh > 1.0) hh = S_(hh, 1.0);
-        else if (hh < 0.0) hh = A_(hh, 1.0);
-    } else {
-        double amp = M_(fp.color_range, tanh(D_(M_(fp.slope, value), fp.scale)));
-        if (fp.attenuation != 0.0) amp = M_(amp, exp(-M_((double)fp.time, fp.attenuation)));
-        hh = asym ? amp : M_(0.5, A_(1.0, amp));
-    }
-    const double hv = M_(256.0, hh);
-    int hue = hv >= 255.0 ? 255 : (hv <= 0.0 ? 0 : (int)hv);
-    double f = dim;
-    if (fp.fade_in_obstacle) {
-        const double cc = (COEF == WG_COEF_TABLE) ? (double)tcc[c] : (m ? p.c2 : p.c2b);
-        f *= pow(cc / p.c2, 0.1);
-    }
-    if (fp.fade) f *= fp.fade_value;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        const double v = (double)lut[hue * 3 + q] * f;
-        int b = (int)(v + 0.5);
-        out[o + q] = (uint8_t)(b > 255 ? 255 : (b < 0 ? 0 : b));
-    }
+    __syncthreads();
+    frame_tile_out(sh, out, w, h, blockIdx.x, blockIdx.y);
 }
 
 // doubles of running state per sampled cell for a plot mode
@@ -158,13 +245,17 @@ wg_status frame_launch(const DevParams &p, const void *phi, const void *psi, int
                        cudaStream_t st)
 {
     const int w = p.nx / fp.size, h = p.ny / fp.size;
-    dim3 grd((w + 127) / 128, h);
+    const FrameFast ff = frame_fast(fp, p);
+    const dim3 grd(frame_tiles_x(w), frame_tiles_y(h)), blk(FT_ROWS, FT_COLS);
+    const auto go = [&](auto kernel, auto *x, auto *y, auto *t) { kernel<<<grd, blk, 0, st>>>(p, x, y, nz, t, lut, fp, ff, acc, out, w, h); };
     if (prec == WG_FP32) {
-        if (coef == WG_COEF_TABLE) k_frame_rgb8<float, WG_COEF_TABLE><<<grd, 128, 0, st>>>(p, (const float *)phi, (const float *)psi, nz, (const float *)tcc, lut, fp, acc, out, w, h);
-        else k_frame_rgb8<float, WG_COEF_MASK><<<grd, 128, 0, st>>>(p, (const float *)phi, (const float *)psi, nz, nullptr, lut, fp, acc, out, w, h);
+        const float *x = (const float *)phi, *y = (const float *)psi, *t = (const float *)tcc;
+        if (coef == WG_COEF_TABLE) go(k_frame_rgb8<float, WG_COEF_TABLE>, x, y, t);
+        else go(k_frame_rgb8<float, WG_COEF_MASK>, x, y, t);
     } else {
-        if (coef == WG_COEF_TABLE) k_frame_rgb8<double, WG_COEF_TABLE><<<grd, 128, 0, st>>>(p, (const double *)phi, (const double *)psi, nz, (const double *)tcc, lut, fp, acc, out, w, h);
-        else k_frame_rgb8<double, WG_COEF_MASK><<<grd, 128, 0, st>>>(p, (const double *)phi, (const double *)psi, nz, nullptr, lut, fp, acc, out, w, h);
+        const double *x = (const double *)phi, *y = (const double *)psi, *t = (const double *)tcc;
+        if (coef == WG_COEF_TABLE) go(k_frame_rgb8<double, WG_COEF_TABLE>, x, y, t);
+        else go(k_frame_rgb8<double, WG_COEF_MASK>, x, y, t);
     }
     WG_CUDA(cudaGetLastError());
     return WG_OK;

@@ -14,6 +14,7 @@
 #include <unordered_map>
 #include <vector>
 #include "wg_batch.h"
+#include "wg_frame.cuh"
 #include "wg_internal.h"
 
 namespace wg {
@@ -23,50 +24,61 @@ struct FrameDev {                // one resident scene in the frame launch
     void *f[4];
     uint32_t *nz;
     int slot;                    // batch slot (its dynamic state says which buffer is phi)
-    int w, h, row_base;
+    int w, h, tile_base;         // its first tile among all scenes'
     unsigned long long out_off;
 };
 
-template <class T>
-__global__ void k_server_frames(const FrameDev *__restrict__ tab, int ntab, const SlotDyn *__restrict__ dyn,
-                                const uint8_t *__restrict__ lut, wg_frame_params fp, uint8_t *__restrict__ out)
+// The palette index in FP64 (no attenuation).
+__device__ __noinline__ int server_hue64(const wg_frame_params &fp, double x)
 {
-    __shared__ int e;
-    if (threadIdx.x == 0) {
-        int lo = 0, hi = ntab - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (tab[mid].row_base <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-        }
-        e = lo;
+    const double value = fp.vshift + fp.vscale * x;
+    const double amp = fp.color_range * tanh(fp.slope * value / fp.scale);
+    const int hue = (int)(256.0 * (0.5 * (1.0 + amp)));
+    return hue > 255 ? 255 : (hue < 0 ? 0 : hue);
+}
+
+// All resident scenes' P_AMPLITUDE frames: a block per tile of pixels of one of them.
+template <class T>
+__global__ void __launch_bounds__(FT_ROWS *FT_COLS) k_server_frames(const FrameDev *__restrict__ tab, int ntab,
+                                                          const SlotDyn *__restrict__ dyn, const uint8_t *__restrict__ lut,
+                                                          const __grid_constant__ wg_frame_params fp,
+                                                          const __grid_constant__ FrameFast ff, uint8_t *__restrict__ out)
+{
+    __shared__ FrameTile sh;
+    int lo = 0, hi = ntab - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tab[mid].tile_base <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
     }
-    __syncthreads();
-    const FrameDev &d = tab[e];
-    const int row = (int)blockIdx.x - d.row_base;
-    if (row >= d.h) return;
-    const SlotDyn dy = dyn[d.slot];
-    const T *phi = (const T *)d.f[2 * dy.pair + dy.cur];
-    const int j = row * fp.size;
-    for (int col = threadIdx.x; col < d.w; col += blockDim.x) {
-        const int i = col * fp.size;
-        uint8_t *o = out + d.out_off + ((size_t)row * d.w + col) * 3;
+    const FrameDev &d = tab[lo];
+    const int tiles = frame_tiles_x(d.w), t = (int)blockIdx.x - d.tile_base, ty = t / tiles, tx = t - ty * tiles;
+    const int row = ty * FT_ROWS + threadIdx.x, col = tx * FT_COLS + threadIdx.y;
+    if (col < d.w && row < d.h) {
+        const SlotDyn dy = dyn[d.slot];
+        const T *phi = (const T *)d.f[2 * dy.pair + dy.cur];
+        const int i = col * fp.size, j = row * fp.size;
+        uint8_t *o = &sh.c[threadIdx.x][3 * threadIdx.y];
         const int m = (d.nz[(size_t)i * d.p.wpitch + (j >> 5)] >> (j & 31)) & 1u;
         if (!(d.p.twospeeds || m)) {
             o[0] = o[1] = o[2] = 0;
-            continue;
-        }
-        const double value = fp.vshift + fp.vscale * (double)phi[(size_t)i * d.p.pitch + j];
-        const double amp = fp.color_range * tanh(fp.slope * value / fp.scale);
-        int hue = (int)(256.0 * (0.5 * (1.0 + amp)));
-        hue = hue > 255 ? 255 : (hue < 0 ? 0 : hue);
-        double f = 1.0;
-        if (fp.fade_in_obstacle) f *= pow((m ? d.p.c2 : d.p.c2b) / d.p.c2, 0.1);
-        if (fp.fade) f *= fp.fade_value;
-        for (int k = 0; k < 3; k++) {
-            const int b = (int)((double)lut[hue * 3 + k] * f + 0.5);
-            o[k] = (uint8_t)(b > 255 ? 255 : (b < 0 ? 0 : b));
+        } else {
+            const T x = phi[(size_t)i * d.p.pitch + j];
+            float err;
+            const float value = amplitude_fast(ff, (float)x, &err);
+            int hue = hue_fast(ff, value, err, false);
+            if (hue < 0) hue = server_hue64(fp, (double)x);
+            if (ff.plain) {
+                for (int k = 0; k < 3; k++) o[k] = lut[hue * 3 + k];
+            } else {
+                const double cc = m ? d.p.c2 : d.p.c2b;
+                float f = fp.fade ? ff.fade : 1.f;
+                if (fp.fade_in_obstacle) f *= powf((float)cc / (float)d.p.c2, 0.1f);
+                if (!colour_fast(lut, hue, f, 8e-7f, o)) frame_colour64(fp, lut, hue, 1.0, cc, d.p.c2, o);
+            }
         }
     }
+    __syncthreads();
+    frame_tile_out(sh, out + d.out_off, d.w, d.h, tx, ty);
 }
 
 static double now_s()
@@ -136,7 +148,7 @@ struct wg_server {
     uint8_t *d_frames[2] = {nullptr, nullptr}, *h_frames[2] = {nullptr, nullptr};
     size_t frames_cap[2] = {0, 0}, frames_bytes[2] = {0, 0};
     FrameDev *d_ftab[2] = {nullptr, nullptr};
-    int ftab_cap[2] = {0, 0}, total_rows[2] = {0, 0}, ntab[2] = {0, 0};
+    int ftab_cap[2] = {0, 0}, total_tiles[2] = {0, 0}, ntab[2] = {0, 0};
     bool layout_dirty[2] = {true, true};  // membership changed since buffer q's layout
     cudaEvent_t ev_start[2] = {nullptr, nullptr}, ev_done[2] = {nullptr, nullptr};
     TickRec rec[2];
@@ -160,7 +172,7 @@ static uint64_t request_bytes(const wg_server *s, const wg_params &p)
 static wg_status server_layout(wg_server *s, int q)
 {
     std::vector<FrameDev> tab;
-    int rows = 0;
+    int tiles = 0;
     unsigned long long off = 0;
     for (int64_t id : s->resident) {
         ServeReq &r = s->reqs[id];
@@ -173,10 +185,10 @@ static wg_status server_layout(wg_server *s, int q)
         d.slot = r.slot;
         d.w = r.w;
         d.h = r.h;
-        d.row_base = rows;
+        d.tile_base = tiles;
         d.out_off = off;
         r.off[q] = off;
-        rows += r.h;
+        tiles += frame_tiles_x(r.w) * frame_tiles_y(r.h);
         off += (unsigned long long)r.w * r.h * 3;
         tab.push_back(d);
     }
@@ -201,7 +213,7 @@ static wg_status server_layout(wg_server *s, int q)
     // the table copy above reads `tab` from pageable memory: the copy is complete when
     // cudaMemcpyAsync returns for pageable sources
     s->frames_bytes[q] = off;
-    s->total_rows[q] = rows;
+    s->total_tiles[q] = tiles;
     s->ntab[q] = (int)tab.size();
     s->layout_dirty[q] = false;
     return WG_OK;
@@ -431,12 +443,15 @@ wg_status wg_server_tick(wg_server *s, int32_t *frames_out)
         }
         WG_CUDA(cudaEventRecord(s->ev_start[q], s->st));
         if ((st = wg_batch_step(s->batch, s->cfg.steps_per_frame))) return st;
+        wg_frame_params steady = s->cfg.frame;
+        steady.attenuation = 0.0;  // the server's frames are not attenuated
+        const FrameFast ff = frame_fast(steady, DevParams());  // P_AMPLITUDE: no energy
         if (s->cfg.precision == WG_FP32)
-            k_server_frames<float><<<s->total_rows[q], 128, 0, s->st>>>(s->d_ftab[q], s->ntab[q], s->batch->d_dyn,
-                                                                        s->d_lut, s->cfg.frame, s->d_frames[q]);
+            k_server_frames<float><<<s->total_tiles[q], dim3(FT_ROWS, FT_COLS), 0, s->st>>>(s->d_ftab[q], s->ntab[q], s->batch->d_dyn, s->d_lut,
+                                                                                 s->cfg.frame, ff, s->d_frames[q]);
         else
-            k_server_frames<double><<<s->total_rows[q], 128, 0, s->st>>>(s->d_ftab[q], s->ntab[q], s->batch->d_dyn,
-                                                                         s->d_lut, s->cfg.frame, s->d_frames[q]);
+            k_server_frames<double><<<s->total_tiles[q], dim3(FT_ROWS, FT_COLS), 0, s->st>>>(s->d_ftab[q], s->ntab[q], s->batch->d_dyn, s->d_lut,
+                                                                                  s->cfg.frame, ff, s->d_frames[q]);
         WG_CUDA(cudaGetLastError());
         s->batch->launches++;
         WG_CUDA(cudaMemcpyAsync(s->h_frames[q], s->d_frames[q], s->frames_bytes[q], cudaMemcpyDeviceToHost, s->st));
