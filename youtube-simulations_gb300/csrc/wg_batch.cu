@@ -357,8 +357,11 @@ static int list_form(const std::vector<const BatchSlotHost *> &hs)
 // Tasks of the pass depth d for the scenes of depth class K (table entries), largest first
 // so that the ticket order balances the warps.  Row chunks: the rows tuned for the scene's
 // size class, or (untuned, fixed depth) sized from the whole list's work, about two tasks
-// per resident team (at least 32 rows), so that no single chunk outlasts the rest of the
-// pass; the short top and bottom segments fill the end.  force_rows > 0 overrides both.
+// per resident team, so that no single chunk outlasts the rest of the pass; the short top and
+// bottom segments fill the end.  A list too small for that (chunks below 32 rows, where the fill
+// costs more than the balance) gives each team about one chunk of at least 8 rows, since its time
+// is that of a chunk: 6 grids of 500x400, 10 updates: 45.6 us in chunks of 32 rows, 39.1 so.
+// force_rows > 0 overrides both.
 static void build_skew_tasks(const wg_batch *b, const std::vector<const BatchSlotHost *> &hs,
                              const std::vector<int> &entries, int d, std::vector<int4> &out, int force_rows = 0)
 {
@@ -366,7 +369,8 @@ static void build_skew_tasks(const wg_batch *b, const std::vector<const BatchSlo
     double rows = 0.0;
     for (const BatchSlotHost *h : hs) rows += (double)batch_skew_tiles(h->dp, d) * (h->prm.nx + 3 * F);
     const int cap = std::max(1, batch_skew_capacity(d, list_form(hs)));
-    const int chunk = std::max(32, std::min(4096, (int)(rows / (2.0 * cap))));
+    const int chunk = rows >= 64.0 * cap ? std::min(4096, (int)(rows / (2.0 * cap)))
+                                         : std::max(8, (int)(rows / cap));
     std::vector<int4> t;
     std::vector<float> cost;
     for (size_t k = 0; k < hs.size(); k++) {
@@ -628,12 +632,13 @@ static void batch_enqueue_frame(wg_batch *b, int n, bool skewed)
                                                           sizeof(T) == 4 ? 1 : 0);
 }
 
-// Depth and row chunk per size class, in two stages: depths 2..4 with the list-wide
+// Depth and row chunk per size class, in two stages: depths 6..2 with the list-wide
 // chunk, then chunks of 32, 64, 128 and 256 rows at the best depth.  Each candidate
 // times one skewed pass over the class's scenes (reading their current fields, writing
 // the other pair, so the state does not change), best of five after one untimed pass;
-// the fastest per update is kept.  Seven candidates per class keep the tuning frame of a
-// server tick short.
+// the fastest per update is kept, a later candidate only if 5% faster (classes run side by
+// side: timed alone, a shallower pass can look a little better and cost the frame 10%).  Nine
+// candidates per class keep the tuning frame of a server tick short.
 // Tuned classes are kept for the process, keyed by device, size class and the kinds of
 // scene in the class (their boundary conditions, the ghost layout, two speeds): a later
 // batch or server whose class holds the same kinds takes that depth and chunk without
@@ -707,9 +712,9 @@ static wg_status batch_autotune(wg_batch *b)
         int4 *dev = nullptr;
         cudaError_t err = cudaSuccess;
         static const int ROWS[] = {32, 64, 128, 256};
-        const int ndepth = 5;  // depths 2..6
+        const int ndepth = 5;  // depths 6..2
         for (int cand = 0; cand < ndepth + 4 && err == cudaSuccess; cand++) {
-            const int K = cand < ndepth ? 2 + cand : best, R = cand < ndepth ? 0 : ROWS[cand - ndepth];
+            const int K = cand < ndepth ? 6 - cand : best, R = cand < ndepth ? 0 : ROWS[cand - ndepth];
             std::vector<int4> tasks;
             build_skew_tasks(b, hs, entries, K, tasks, R);
             const int nt = (int)tasks.size();
@@ -737,7 +742,7 @@ static wg_status batch_autotune(wg_batch *b)
             if (err == cudaSuccess) err = cudaStreamSynchronize(b->st);  // tasks outlives its copy
             const double per = ms / K;
             if (R == 0 || per < b->tune_ms[c * 8 + K]) b->tune_ms[c * 8 + K] = per;
-            if (per < best_ms) {
+            if (per < 0.95 * best_ms) {
                 best_ms = per;
                 best = K;
                 best_rows = R;

@@ -16,6 +16,7 @@
 // Periodic and VPER_HABS boundaries (which read the opposite side of the grid) and
 // Neumann gathers use the single-step kernel.
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
 #include <map>
 #include <mutex>
@@ -721,8 +722,7 @@ __device__ __forceinline__ void skew_strip(const DevParams &p, const TbArgs &a, 
     int m = m0 + 2 * s_first - 4 * w;
     if (P > 1)
         for (int s = 0; s < s_first; s++) team_sync();
-#pragma unroll 1
-    for (int s = s_first; s <= s_last; s++, m += 2) {
+    const auto step = [&](auto edge) {
         if (w == 0) cp_async_wait<SK_IN - 2>();  // the rows of step s have landed
         unsigned act[3] = {0xFu, 0xFu, 0xFu};  // rows m-2, m-1, m
         f2 T[3][2];
@@ -748,14 +748,14 @@ __device__ __forceinline__ void skew_strip(const DevParams &p, const TbArgs &a, 
             te[2] = my1[SM::TCE + tcur];
         }
         f2 xo[2][2], vo[2][2];
-        if (EDGE) {
-            // the full rules only where the step computes row 0, nx-1 or the point source
+        constexpr int E = decltype(edge)::value;
+        if constexpr (E == 3) {
             const bool full = p.osc_topbot || (m >= 0 && m <= 2) || (m >= p.nx - 1 && m <= p.nx + 1) ||
                               (p.src_on && m >= p.src_i && m <= p.src_i + 2);
             if (full) skew_step<COEF, PL, 2, INL>(p, a, kk, ed, m, w, gj0, in, T, te, act, q, xo, vo);
             else skew_step<COEF, PL, 1, INL>(p, a, kk, ed, m, w, gj0, in, T, te, act, q, xo, vo);
         } else {
-            skew_step<COEF, PL, 0, INL>(p, a, kk, ed, m, w, gj0, in, T, te, act, q, xo, vo);
+            skew_step<COEF, PL, E, INL>(p, a, kk, ed, m, w, gj0, in, T, te, act, q, xo, vo);
         }
         if (!last) {
             float *out = out_lo + out_at;
@@ -780,6 +780,33 @@ __device__ __forceinline__ void skew_strip(const DevParams &p, const TbArgs &a, 
         tcur = tcur == (SM::NT - 1) * 64 ? 0 : tcur + 64;
         if (w == 0) issue();  // into slots that no warp reads any more
         if (P > 1) team_sync();
+    };
+    if (!EDGE || !INL) {
+        // EDGE (3): the full rules only where a step computes row 0, nx-1 or the point source
+#pragma unroll 1
+        for (int s = s_first; s <= s_last; s++, m += 2) step(std::integral_constant<int, EDGE ? 3 : 0>());
+    } else {
+        // The same in loops of their own: as branches of one loop the two forms cost a batch's masked
+        // strips 1.7 times the inner strip's instructions instead of 1.45 (64 scenes of 1000x120,
+        // mirror: 113 to 99 us for 10 updates).  (Single grids' table forms spill more this way:
+        // 1172 to 1058 Gcell/s on 3840x2160.)
+        const auto next_full = [&](int mm) {
+            if (p.osc_topbot) return mm;
+            int n = 0x7fffffff;
+            if (p.src_on && mm <= p.src_i + 2) n = p.src_i;
+            if (mm <= p.nx + 1) n = min(n, p.nx - 1);
+            return mm <= 2 ? min(n, 0) : n;
+        };
+        const int m_last = m + 2 * (s_last - s_first);
+        while (m <= m_last) {
+            const int mf = min(next_full(m), m_last + 1);
+#pragma unroll 1
+            for (; m < mf; m += 2) step(std::integral_constant<int, 1>());
+            if (m <= m_last && m >= next_full(m)) {
+                step(std::integral_constant<int, 2>());
+                m += 2;
+            }
+        }
     }
     if (P > 1)
         for (int s = s_last + 1; s < nsteps; s++) team_sync();
@@ -984,17 +1011,24 @@ static wg_status skew_tasks(wg_scene *s, int K, int L, const int4 **tasks, int *
 }
 
 // ---------------------------------------------------------------------------
-// Skewed passes over a batch of scenes (mask coefficients, FP32).  Persistent teams take
-// tasks from a ticket counter: table entry, first column of the tile (shifted tiling),
+// Skewed passes over a batch of scenes (mask coefficients, FP32).  Each team takes the task of
+// its block, then, from a longer list, tasks by a ticket counter: table entry, first column of the tile (shifted tiling),
 // rows i_s | i_e << 16, kind (0 inner, 1 EDGE, 3 periodic in the ghost layout).  The scene's
 // parameters are staged in the team's shared memory.  Pass q of a frame reads pair
 // (pair ^ q) of the scene and writes the other pair.  Oscillating values and source
 // increments are computed inline at update time + toff + level.
+//
+// The first task goes by block because a pass's blocks are resident early, where the pass before
+// left room: taken by ticket, a short list's tasks fell on the SMs unevenly (6 grids of 500x400,
+// 10 updates, mirror: 53.5 us by ticket with 15 warps per SM, 70 with 21; 39.1 now).  15 warps
+// per SM, the most that 128 registers allow, measured 10-15% slower than 21 on long lists, although
+// the general form spills (64 scenes of 1000x896, mirror: 630 to 512 us; 192 scenes of 128 to
+// 512 a side, absorbing: 333 to 285 us for 10 updates).
 // ---------------------------------------------------------------------------
 static_assert(sizeof(DevParams) % 4 == 0, "DevParams is copied as 32-bit words");
 
 template <int P, int PL>
-__global__ void __launch_bounds__(32 * P, 16 / P)
+__global__ void __launch_bounds__(32 * P, P == 1 ? 16 : skew_min_blocks(P))
     k_batch_skew(const SlotDev *__restrict__ tab, const SlotDyn *__restrict__ dyn, const int4 *__restrict__ tasks,
                  const int *__restrict__ ntasks, int *__restrict__ ticket, int K, int q, int toff)
 {
@@ -1003,21 +1037,22 @@ __global__ void __launch_bounds__(32 * P, 16 / P)
     __shared__ int s_ticket;
     const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     float *shm = reinterpret_cast<float *>(skew_smem);
-    pdl_wait();  // launched by launch_pdl: the previous pass (or ghost refresh) has completed
-    pdl_trigger();
+    // The lists and the scenes' parameters do not change within a frame, and the first pass of
+    // a frame is not launched early: they are read before the wait for the previous pass.
     const int n = *ntasks, H = (K + 3) & ~3;
-    for (;;) {
-        __syncthreads();  // every warp is done with the previous task
-        if (threadIdx.x == 0) s_ticket = atomicAdd(ticket, 1);
-        __syncthreads();
-        const int t = s_ticket;
-        if (t >= n) break;
+    if (n == 0) pdl_wait();  // (so that the pass after this one still waits for the one before)
+    int t = blockIdx.x;  // the first tasks by block, so that they spread over the SMs; then by ticket
+    for (bool first = true; t < n; first = false) {
         const int4 d = tasks[t];
         const SlotDev &sd = tab[d.x];
         {
             const int *src = reinterpret_cast<const int *>(&sd.p);
             int *dst = reinterpret_cast<int *>(&p);
             for (int k = threadIdx.x; k < (int)(sizeof(DevParams) / 4); k += 32 * P) dst[k] = src[k];
+        }
+        if (first) {
+            pdl_wait();
+            pdl_trigger();
         }
         __syncthreads();
         const SlotDyn dy = dyn[sd.slot];
@@ -1056,6 +1091,11 @@ __global__ void __launch_bounds__(32 * P, 16 / P)
         else
             skew_strip<WG_COEF_MASK, PL, P, false, true>(p, a, K, i_s, i_e, gj0, lane, w, shm, lo, hi, -gr, p.nx + gr, -gc,
                                                          p.ny + gc);
+        if (n <= (int)gridDim.x) break;
+        __syncthreads();  // every warp is done with the task
+        if (threadIdx.x == 0) s_ticket = (int)gridDim.x + atomicAdd(ticket, 1);
+        __syncthreads();
+        t = s_ticket;
     }
 }
 
