@@ -1,0 +1,52 @@
+"""Downloads into page-locked rows, which the forming kernel writes in place in whole lines: rows
+that start anywhere in a line, either row alone, grids of one lane to several blocks, both
+precisions, scenes and batches; the same bits as through pageable rows, and nothing beside them."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from youtube_simulations_gb300 import params as P
+from youtube_simulations_gb300 import wavegpu as W
+
+pytestmark = pytest.mark.gpu
+
+
+def pinned(n, offset, dt):
+    """An array of n cells, `offset` cells into page-locked memory, and the whole of it (filled with 7)."""
+    whole = torch.empty((n + 2 * offset + 40,), dtype=dt, pin_memory=True).numpy()
+    whole[:] = 7.0
+    return whole[offset:offset + n], whole
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 3), (3, 8), (5, 33), (31, 64), (64, 131), (67, 257)])
+@pytest.mark.parametrize("prec,native", [(P.FP32, True), (P.FP32, False), (P.FP64, False)])
+@pytest.mark.parametrize("offsets", [(0, 0), (1, 3), (17, 30)])
+def test_page_locked_rows(nx, ny, prec, native, offsets):
+    rng = np.random.default_rng(nx + ny)
+    n = nx * ny
+    p = P.make_params(nx, ny, b_cond=P.BC_DIRICHLET, courant=0.1)
+    xy = np.ones(n, np.int16)
+    f = rng.standard_normal(n), rng.standard_normal(n)
+    dt = torch.float32 if native else torch.float64
+    code = P.FP32 if native else P.FP64
+    with W.Scene(p, prec, P.COEF_MASK) as s, W.Batch(prec) as b:
+        s.upload(*f, xy)
+        s.step(1)
+        slot = b.add(p, *f, xy)
+        b.step(1)
+        ref = s.download(native=native)
+        calls = [lambda x, y: W.lib().wg_scene_download(s.h, x, y, code)]
+        if not native:
+            calls.append(lambda x, y: W.lib().wg_batch_download(b.h, slot, x, y))
+        for call in calls:
+            for use in ((True, True), (True, False), (False, True)):
+                rows = [pinned(n, o, dt) for o in offsets]
+                W.check(call(*(ctypes.c_void_p(r.ctypes.data) if u else None for (r, _), u in zip(rows, use))))
+                for (r, whole), u, o, want in zip(rows, use, offsets, ref):
+                    assert np.array_equal(r, want) if u else np.all(r == 7.0)
+                    assert np.all(whole[:o] == 7.0) and np.all(whole[o + n:] == 7.0)
+        both, _ = pinned(n, 1, dt)  # the same rows twice: psi's copy comes last
+        W.check(calls[0](both.ctypes.data, both.ctypes.data))
+        assert np.array_equal(both, ref[1])

