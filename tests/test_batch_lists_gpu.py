@@ -22,7 +22,7 @@ def instance(k, nx, ny, bc):
 
 
 @pytest.mark.parametrize("bc", [P.BC_DIRICHLET, P.BC_ABSORBING, P.BC_PERIODIC])
-@pytest.mark.parametrize("count,nx,ny", [(1, 9, 40), (1, 131, 257), (3, 33, 240), (40, 70, 129), (420, 61, 250)])
+@pytest.mark.parametrize("count,nx,ny", [(2, 4, 9), (3, 6, 13), (1, 9, 40), (1, 131, 257), (3, 33, 240), (40, 70, 129), (420, 61, 250)])
 @pytest.mark.parametrize("mode", [3, 6, -1])
 def test_lists_of_every_length(bc, count, nx, ny, mode):
     with W.Batch(P.FP32) as b:

@@ -231,20 +231,19 @@ __global__ void __launch_bounds__(128, 4) k_batch_step64(const BatchHdr *__restr
     }
 }
 
-// Ghost cells of the input pair of pass q for the wrapped scenes of depth class K (K < 0:
-// every wrapped scene, the current pair): each ghost cell of both fields takes the value of
+// Ghost cells of every wrapped scene's current pair, when its fields do not come from a skewed
+// pass (which writes them beside its cells): each ghost cell of both fields takes the value of
 // the real cell it wraps to.  Ghost cells are written and real cells read, so blocks need
 // no ordering.  Block (x, y): table entry x, a share y of its ghost cells.
 __global__ void k_batch_ghosts(const BatchHdr *__restrict__ hdr, const SlotDev *__restrict__ tab,
-                               const SlotDyn *__restrict__ dyn, int K, int q)
+                               const SlotDyn *__restrict__ dyn)
 {
     const int e = blockIdx.x;
     if (e >= hdr->nactive) return;
     const SlotDev &sd = tab[e];
-    if (!sd.wrap || (K >= 0 && sd.skew_k != K)) return;
-    const SlotDyn dy = dyn[sd.slot];
-    const int pin = K < 0 ? dy.pair : dy.pair ^ (q & 1);
-    float *f0 = (float *)sd.f[2 * pin], *f1 = (float *)sd.f[2 * pin + 1];
+    if (!sd.wrap) return;
+    const int pair = dyn[sd.slot].pair;
+    float *f0 = (float *)sd.f[2 * pair], *f1 = (float *)sd.f[2 * pair + 1];
     const int nx = sd.p.nx, ny = sd.p.ny, pitch = sd.p.pitch;
     constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
     const int wide = ny + 2 * GC, ncol = 2 * GC * nx, total = ncol + 2 * GR * wide;
@@ -491,7 +490,6 @@ wg_status batch_refresh_table(wg_batch *b)
         }
     }
     if (plain > 0) sig |= 1u;
-    if (nwrap > 0) sig |= 1u << 8;  // ghost refreshes in the branches
     if ((int)tab.size() > b->tab_cap) {
         if (b->d_tab) cudaFree(b->d_tab);
         b->d_tab = nullptr;
@@ -524,6 +522,7 @@ wg_status batch_refresh_table(wg_batch *b)
     b->plain_tiles = plain;
     b->skew_scenes = nskew;
     b->wrap_scenes = nwrap;
+    b->ghosts_ok = false;  // the table may hold new scenes, or scenes that took single updates
     b->tab_slot = tab_slot;
     // the task lists in use follow the new table
     std::vector<std::pair<int, int>> keys;
@@ -611,8 +610,6 @@ static void batch_enqueue_frame(wg_batch *b, int n, bool skewed)
             for (int q = 0; q < P; q++) {
                 const int d = batch_pass_depth(n, P, q);
                 const BatchSkewList &L = b->lists.at({K, d});
-                if (b->graph_sig & (1u << 8))  // the wrapped scenes' ghosts of this pass's input pair
-                    k_batch_ghosts<<<dim3(std::max(b->tab_cap, 1), 8), 256, 0, ss>>>(b->d_hdr, b->d_tab, b->d_dyn, K, q);
                 launch_batch_skew(d, L.form, b->d_tab, b->d_dyn, L.dev, b->d_skew_n + L.index, b->d_ticket + ti++, q, toff, ss);
                 toff += d;
             }
@@ -701,7 +698,7 @@ static wg_status batch_autotune(wg_batch *b)
         if (hs.empty()) continue;
         if (b->tune_ms.empty()) b->tune_ms.assign(BATCH_CLASSES * 8, 0.0);
         if (!ghosts) {  // the wrapped scenes' ghosts of their current pair, read by the timed passes
-            k_batch_ghosts<<<dim3(std::max(b->nactive, 1), 8), 256, 0, b->st>>>(b->d_hdr, b->d_tab, b->d_dyn, -1, 0);
+            k_batch_ghosts<<<dim3(std::max(b->nactive, 1), 8), 256, 0, b->st>>>(b->d_hdr, b->d_tab, b->d_dyn);
             b->launches++;
             ghosts = true;
         }
@@ -958,11 +955,17 @@ wg_status wg_batch_step(wg_batch *b, int32_t nsteps)
         if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
         it = b->graphs.emplace(nsteps, ge).first;
     }
+    if (skewed && b->wrap_scenes > 0 && !b->ghosts_ok) {
+        k_batch_ghosts<<<dim3(b->nactive, 8), 256, 0, b->st>>>(b->d_hdr, b->d_tab, b->d_dyn);
+        WG_CUDA(cudaGetLastError());
+        b->launches++;
+    }
     WG_CUDA(cudaGraphLaunch(it->second, b->st));
+    b->ghosts_ok = skewed;  // (nsteps >= 2: every depth class takes at least one pass)
     long long n = 1;  // the advance kernel
     if (!skewed || (b->graph_sig & 1u)) n += nsteps;
     if (skewed)
-        for (int K : batch_groups(b)) n += batch_passes(nsteps, K) * ((b->graph_sig & (1u << 8)) ? 2 : 1);
+        for (int K : batch_groups(b)) n += batch_passes(nsteps, K);
     b->launches += n;
     return WG_OK;
 }

@@ -140,6 +140,7 @@ struct wg_batch {
     cudaEvent_t ev_fork = nullptr, ev_join[wg::BATCH_GROUPS] = {};
     unsigned graph_sig = 0;                               // depth classes present (bit K), plain chain (bit 0)
     int plain_tiles = 0, skew_scenes = 0, wrap_scenes = 0;
+    bool ghosts_ok = false;                               // the wrapped scenes' current pairs hold their ghosts
     std::vector<int> tab_slot;                            // slot of each table entry
     int *d_tune_ticket = nullptr;                         // tickets of the autotuner's passes
     std::vector<double> tune_ms;                          // last autotune: ms per update, [class * 8 + K]
