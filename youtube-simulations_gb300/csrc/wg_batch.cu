@@ -231,10 +231,35 @@ __global__ void __launch_bounds__(128, 4) k_batch_step64(const BatchHdr *__restr
     }
 }
 
+// Ghost cells t0, t0 + nt, .. of one grid: each takes the value of the real cell it wraps to, in
+// both fields (f1 may be NULL).  Ghost cells are written and real cells read, so blocks need no
+// ordering.
+__device__ __forceinline__ void ghost_fill(float *f0, float *f1, int nx, int ny, int pitch, long long t0, long long nt)
+{
+    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
+    const int wide = ny + 2 * GC, ncol = 2 * GC * nx;
+    const long long total = ncol + 2LL * GR * wide;
+    for (long long t = t0; t < total; t += nt) {
+        int i, j;
+        if (t < ncol) {  // the ghost columns of the real rows
+            i = (int)t / (2 * GC);
+            const int g = (int)t - i * 2 * GC;
+            j = g < GC ? g - GC : ny + g - GC;
+        } else {  // the ghost rows, over the extended width
+            const int u = (int)(t - ncol), rg = u / wide;
+            j = u - rg * wide - GC;
+            i = rg < GR ? rg - GR : nx + rg - GR;
+        }
+        const int si = ((i % nx) + nx) % nx, sj = ((j % ny) + ny) % ny;
+        const long long d = (long long)i * pitch + j, s = (long long)si * pitch + sj;
+        f0[d] = f0[s];
+        if (f1) f1[d] = f1[s];
+    }
+}
+
 // Ghost cells of every wrapped scene's current pair, when its fields do not come from a skewed
-// pass (which writes them beside its cells): each ghost cell of both fields takes the value of
-// the real cell it wraps to.  Ghost cells are written and real cells read, so blocks need
-// no ordering.  Block (x, y): table entry x, a share y of its ghost cells.
+// pass (which writes them beside its cells).  Block (x, y): table entry x, a share y of its
+// ghost cells.
 __global__ void k_batch_ghosts(const BatchHdr *__restrict__ hdr, const SlotDev *__restrict__ tab,
                                const SlotDyn *__restrict__ dyn)
 {
@@ -243,26 +268,19 @@ __global__ void k_batch_ghosts(const BatchHdr *__restrict__ hdr, const SlotDev *
     const SlotDev &sd = tab[e];
     if (!sd.wrap) return;
     const int pair = dyn[sd.slot].pair;
-    float *f0 = (float *)sd.f[2 * pair], *f1 = (float *)sd.f[2 * pair + 1];
-    const int nx = sd.p.nx, ny = sd.p.ny, pitch = sd.p.pitch;
-    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
-    const int wide = ny + 2 * GC, ncol = 2 * GC * nx, total = ncol + 2 * GR * wide;
-    for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < total; t += gridDim.y * blockDim.x) {
-        int i, j;
-        if (t < ncol) {  // the ghost columns of the real rows
-            i = t / (2 * GC);
-            const int g = t - i * 2 * GC;
-            j = g < GC ? g - GC : ny + g - GC;
-        } else {  // the ghost rows, over the extended width
-            const int u = t - ncol, rg = u / wide;
-            j = u - rg * wide - GC;
-            i = rg < GR ? rg - GR : nx + rg - GR;
-        }
-        const int si = ((i % nx) + nx) % nx, sj = ((j % ny) + ny) % ny;
-        const long long d = (long long)i * pitch + j, s = (long long)si * pitch + sj;
-        f0[d] = f0[s];
-        f1[d] = f1[s];
-    }
+    ghost_fill((float *)sd.f[2 * pair], (float *)sd.f[2 * pair + 1], sd.p.nx, sd.p.ny, sd.p.pitch,
+               blockIdx.y * blockDim.x + threadIdx.x, gridDim.y * blockDim.x);
+}
+
+// The same of one grid (scenes).
+__global__ void k_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch)
+{
+    ghost_fill(f0, f1, nx, ny, pitch, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
+void launch_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch, cudaStream_t st)
+{
+    const long long total = 2LL * BATCH_GHOST_COLS * nx + 2LL * BATCH_GHOST_ROWS * (ny + 2 * BATCH_GHOST_COLS);
+    k_grid_ghosts<<<(unsigned)std::min(608LL, (total + 127) / 128), 128, 0, st>>>(f0, f1, nx, ny, pitch);
 }
 
 // The ghost words and rows of a wrapped scene's active plane: one thread per word of rows
@@ -292,6 +310,11 @@ __global__ void k_act_ghosts(uint32_t *act, int wpitch, int nx, int ny)
         v |= x << bit;
     }
     act[base] = v;
+}
+void launch_act_ghosts(uint32_t *act, int wpitch, int nx, int ny, cudaStream_t st)
+{
+    const int words = (ny + BATCH_GHOST_COLS + 31) / 32 + 1, rows = nx + 2 * BATCH_GHOST_ROWS;
+    k_act_ghosts<<<dim3((words + 63) / 64, rows), 64, 0, st>>>(act, wpitch, nx, ny);
 }
 
 // skewed: the frame ran the skewed passes of the scenes with a depth class.  pairs: FP32
@@ -879,8 +902,7 @@ wg_status wg_batch_add(wg_batch *b, const wg_params *p, const double *phi, const
     WG_CUDA(cudaMemcpyAsync(stage, xy, n * sizeof(int16_t), cudaMemcpyHostToDevice, b->st));
     launch_pack_mask(p->nx, p->ny, h.dp.wpitch, (const int16_t *)stage, h.act, h.nz, b->st);
     if (h.wrap) {  // the mask's ghost words and rows, once (the mask does not change)
-        const int words = (p->ny + BATCH_GHOST_COLS + 31) / 32 + 1, rows = p->nx + 2 * BATCH_GHOST_ROWS;
-        k_act_ghosts<<<dim3((words + 63) / 64, rows), 64, 0, b->st>>>(h.act, h.dp.wpitch, p->nx, p->ny);
+        launch_act_ghosts(h.act, h.dp.wpitch, p->nx, p->ny, b->st);
         b->launches++;
     }
     double *dstage = (double *)stage;

@@ -73,6 +73,8 @@ void batch_skew_plan(const DevParams &p, int entry, int K, int rows, std::vector
 void launch_batch_skew(int K, int form, const SlotDev *tab, const SlotDyn *dyn, const int4 *tasks, const int *ntasks,
                        int *ticket, int q, int toff, cudaStream_t st);
 bool batch_skew_ok(const wg_params &p, int prec);
+void launch_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch, cudaStream_t st);  // f1 may be NULL
+void launch_act_ghosts(uint32_t *act, int wpitch, int nx, int ny, cudaStream_t st);
 bool batch_wrap_ok(const wg_params &p, int prec);   // periodic scenes the skewed passes take (ghost layout)
 
 wg_status batch_refresh_table(::wg_batch *b);

@@ -415,6 +415,7 @@ extern "C" wg_status wg_scene_build_domain(wg_scene *s, int32_t domain, double l
     s->has_ghosts = nrec > 0;
     s->xy_host.clear();
     s->has_mask = true;
+    s->mask_ghosts_ok = false;
     s->tb_k = 0;  // autotuned again for the new geometry
     return WG_OK;
 }

@@ -6,9 +6,11 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <string>
 #include <vector>
 #include "wg_internal.h"
 #include "wg_scene.h"
+#include "wg_batch.h"
 
 using namespace wg;
 
@@ -67,17 +69,27 @@ wg_status scene_alloc_dense_stage(wg_scene *s, size_t bytes)
     return WG_OK;
 }
 
+void *scene_field_base(const wg_scene *s, void *f) { return f ? (char *)f - s->field_off * s->esz : nullptr; }
+
+wg_status scene_alloc_field(wg_scene *s, void **f)
+{
+    void *m = nullptr;
+    WG_CUDA(cudaMalloc(&m, s->field_bytes));
+    *f = (char *)m + s->field_off * s->esz;
+    WG_CUDA(cudaMemsetAsync(m, 0, s->field_bytes, s->st));
+    return WG_OK;
+}
+
 size_t scene_device_bytes(const wg_params &p, int prec, int coef)
 {
-    const size_t esz = prec == WG_FP32 ? 4 : 8;
-    const size_t pitch = pitch_for(p.ny, (int)esz), wp = (pitch + 31) / 32;
-    size_t b = 2 * (size_t)p.nx * pitch * esz;          // phi, psi
-    b += 2 * (size_t)p.nx * wp * 4;                     // act, nz planes
+    const BatchLayout L = batch_layout(p, prec);
+    size_t b = 2 * L.field_bytes;                       // phi, psi
+    b += 2 * L.mask_bytes;                              // act, nz planes
     if (coef == WG_COEF_TABLE) {
-        b += (size_t)p.nx * pitch * esz;                // tcc
-        if (p.b_cond == WG_BC_ABSORBING || p.b_cond == WG_BC_VPER_HABS) b += (size_t)p.nx * pitch * esz;  // tc
+        b += L.field_bytes;                             // tcc
+        if (p.b_cond == WG_BC_ABSORBING || p.b_cond == WG_BC_VPER_HABS) b += L.field_bytes;  // tc
     }
-    if (prec == WG_FP32) b += 2 * (size_t)p.nx * pitch * esz;  // FP32: the output pair of every update
+    if (prec == WG_FP32) b += 2 * L.field_bytes;        // FP32: the output pair of every update
     b += (size_t)p.nx * 2 * sizeof(double2) + (p.nx + 8) * sizeof(double) + 64;  // energy scratch
     return b;
 }
@@ -195,6 +207,7 @@ template <class T>
 static wg_status single_update(wg_scene *s)
 {
     s->time++;
+    s->ghosts_ok = false;
     const bool recs = s->nrec > 0;
     FastArgs<T> a = fast_args<T>(s, recs ? 0 : 1);
     s->launches += launch_step_fast<T>(s->dp, a, s->coef, s->time, s->st);
@@ -223,7 +236,13 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
         return WG_ERR_STATE;
     }
     const int k = s->tb_k;
-    const bool tb = k > 1 && tb_supported(s) && !s->probe_n;  // probes sample every update
+    // probes sample every update; the TMA tiles do not wrap
+    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1);
+    // a recorded call may be replayed after other calls have changed the fields or the mask: it
+    // fills the ghosts itself, and leaves them to the next call
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (tb && s->wrap) WG_CUDA(cudaStreamIsCapturing(s->st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) s->ghosts_ok = s->mask_ghosts_ok = false;
     if (tb) {
         wg_status st = tb_prepare(s, nsteps);
         if (st) return st;
@@ -241,6 +260,7 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
             nsteps--;
         }
     }
+    if (cap != cudaStreamCaptureStatusNone) s->ghosts_ok = s->mask_ghosts_ok = false;
     WG_CUDA(cudaGetLastError());
     return WG_OK;
 }
@@ -299,7 +319,13 @@ wg_status wg_scene_create(const wg_params *p, int32_t precision, int32_t coef_mo
     s->prec = precision;
     s->coef = coef_mode;
     s->esz = precision == WG_FP32 ? 4 : 8;
-    s->pitch = pitch_for(p->ny, (int)s->esz);
+    const BatchLayout L = batch_layout(*p, precision);
+    s->wrap = batch_wrap_ok(*p, precision);
+    s->pitch = L.pitch;
+    s->field_off = L.field_off;
+    s->mask_off = L.mask_off;
+    s->field_bytes = L.field_bytes;
+    s->mask_bytes = L.mask_bytes;
     s->dp = make_dev_params(*p, s->pitch);
     if (stream) s->st = (cudaStream_t)stream;
     else {
@@ -307,25 +333,23 @@ wg_status wg_scene_create(const wg_params *p, int32_t precision, int32_t coef_mo
         if (e != cudaSuccess) { delete s; return cuda_fail(e, "cudaStreamCreate"); }
         s->own_stream = true;
     }
-    const size_t fb = (size_t)p->nx * s->pitch * s->esz, mb = (size_t)p->nx * s->dp.wpitch * 4;
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
-        e = cudaMalloc(&s->f[k], fb);
-        if (e == cudaSuccess) e = cudaMemsetAsync(s->f[k], 0, fb, s->st);
-        if (e == cudaSuccess && precision == WG_FP32) e = cudaMalloc(&s->g[k], fb);
-        if (e == cudaSuccess && precision == WG_FP32) e = cudaMemsetAsync(s->g[k], 0, fb, s->st);
+    bool ok = true;
+    for (int k = 0; k < 2 && ok; k++)
+        ok = scene_alloc_field(s, &s->f[k]) == WG_OK && (precision != WG_FP32 || scene_alloc_field(s, &s->g[k]) == WG_OK);
+    if (ok && coef_mode == WG_COEF_TABLE)
+        ok = scene_alloc_field(s, &s->tcc) == WG_OK &&
+             ((p->b_cond != WG_BC_ABSORBING && p->b_cond != WG_BC_VPER_HABS) || scene_alloc_field(s, &s->tc) == WG_OK);
+    if (!ok) {
+        const std::string msg = wg_last_error();
+        wg_scene_destroy(s);
+        set_error("%s", msg.c_str());
+        return WG_ERR_CUDA;
     }
-    if (e == cudaSuccess) e = cudaMalloc(&s->act, mb);
-    if (e == cudaSuccess) e = cudaMalloc(&s->nz, mb);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->act, 0, mb, s->st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->nz, 0, mb, s->st);
-    if (e == cudaSuccess && coef_mode == WG_COEF_TABLE) {
-        e = cudaMalloc(&s->tcc, fb);
-        if (e == cudaSuccess) e = cudaMemsetAsync(s->tcc, 0, fb, s->st);
-        if (e == cudaSuccess && (p->b_cond == WG_BC_ABSORBING || p->b_cond == WG_BC_VPER_HABS)) {
-            e = cudaMalloc(&s->tc, fb);
-            if (e == cudaSuccess) e = cudaMemsetAsync(s->tc, 0, fb, s->st);
-        }
+    cudaError_t e = cudaSuccess;
+    for (uint32_t **m : {&s->act, &s->nz}) {
+        if (e == cudaSuccess) e = cudaMalloc(m, s->mask_bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(*m, 0, s->mask_bytes, s->st);
+        if (*m) *m += s->mask_off;
     }
     if (e == cudaSuccess) e = cudaMalloc(&s->ebot, p->nx * sizeof(double2));
     if (e == cudaSuccess) e = cudaMalloc(&s->etop, p->nx * sizeof(double2));
@@ -349,9 +373,10 @@ wg_status wg_scene_destroy(wg_scene *s)
 {
     if (!s) return WG_OK;
     if (s->st) cudaStreamSynchronize(s->st);
-    for (auto &f : s->f) if (f) cudaFree(f);
-    for (auto &g : s->g) if (g) cudaFree(g);
-    void *dev[] = {s->act, s->nz, s->tcc, s->tc, s->tg, s->nidx, s->nw, s->ebot, s->etop, s->eout, s->dcount,
+    void *fields[] = {s->f[0], s->f[1], s->g[0], s->g[1], s->tcc, s->tc};
+    for (void *f : fields) if (f) cudaFree(scene_field_base(s, f));
+    for (uint32_t *m : {s->act, s->nz}) if (m) cudaFree(m - s->mask_off);
+    void *dev[] = {s->tg, s->nidx, s->nw, s->ebot, s->etop, s->eout, s->dcount,
                    s->dstage, s->rgb, s->lut, s->bv_osc, s->bv_src, s->dflag, s->facc, s->probe_cells, s->probe_buf,
                    s->nrec_dev};
     for (void *d : dev) if (d) cudaFree(d);
@@ -423,6 +448,7 @@ wg_status wg_scene_upload(wg_scene *s, const double *phi, const double *psi, con
     s->time = 0;
     s->uploaded = true;
     s->has_mask = true;
+    s->ghosts_ok = s->mask_ghosts_ok = false;
     return WG_OK;
 }
 
@@ -435,6 +461,7 @@ wg_status wg_scene_upload_state(wg_scene *s, const void *phi, const void *psi, i
     if (!s->has_mask) { set_error("upload or build the mask first"); return WG_ERR_STATE; }
     if (host_precision != WG_FP32 && host_precision != WG_FP64) { set_error("unknown host precision"); return WG_ERR_INVALID; }
     s->uploaded = true;
+    s->ghosts_ok = false;
     if (s->prec == WG_FP32) {  // stream-ordered for FP32 host rows, as for same-precision copies below
         if (host_precision == WG_FP32) return upload_state32<float>(s, (const float *)phi, (const float *)psi, false);
         return upload_state32<double>(s, (const double *)phi, (const double *)psi, true);

@@ -22,6 +22,12 @@ struct wg_scene {
     void *f[2] = {nullptr, nullptr};  // f[cur] = phi (level t), f[1-cur] = psi (FP64) or the velocity (FP32)
     void *g[2] = {nullptr, nullptr};  // FP32: the output pair of every update and blocked pass
     int cur = 0;
+    // A periodic FP32 scene that takes skewed passes lies in the ghost layout of batches: the pointers
+    // to its fields, tables and masks address cell (0, 0), field_off cells and mask_off words into
+    // allocations of field_bytes and mask_bytes.  ghosts_ok: the current fields hold their
+    // ghosts; mask_ghosts_ok: the active plane and tcc do.
+    bool wrap = false, ghosts_ok = false, mask_ghosts_ok = false;
+    size_t field_off = 0, mask_off = 0, field_bytes = 0, mask_bytes = 0;
     uint32_t *act = nullptr, *nz = nullptr;
     int has_ghosts = 0;
     std::vector<int16_t> xy_host;
@@ -60,6 +66,8 @@ struct wg_scene {
 
 namespace wg {
 wg_status scene_alloc_dense_stage(wg_scene *s, size_t bytes);
+void *scene_field_base(const wg_scene *s, void *f);  // the allocation of a field, or nullptr
+wg_status scene_alloc_field(wg_scene *s, void **f);  // zeroed, in the scene's layout
 size_t scene_device_bytes(const wg_params &p, int prec, int coef);
 template <class T> wg_status scene_step_impl(wg_scene *s, int nsteps);
 // temporal blocking (wg_tb.cu)

@@ -840,6 +840,78 @@ __global__ void __launch_bounds__(32 * P, skew_min_blocks(P))
         skew_strip<COEF, PL, P, false, false>(p, a, K, t.y, t.z, gj0, lane, w, shm, lo, hi, 0, p.nx, 0, p.ny);
 }
 
+// The ghost cells that mirror the rows [i_s, i_e) and columns [lo, hi) of a wrapped scene's new
+// fields, by the team that stored them: a cell within BATCH_GHOST_COLS of the left or right edge or
+// BATCH_GHOST_ROWS of the top or bottom one goes to every place of the extended grid that wraps to
+// it.  (The last group of four columns may reach past ny-1; the cells it stores there are the
+// same values.)  A kernel before each pass did this over the whole batch, 22 us with 48 scenes, and
+// kept passes from overlapping: 48 scenes of 256 to 960 a side, half of them periodic, 10 updates:
+// 224 to 195 us.
+__device__ __noinline__ void skew_images(float *f0, float *f1, int nx, int ny, int pitch, int i_s, int i_e, int lo, int hi,
+                                         int t0, int nt)
+{
+    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
+    // cells t0, t0 + nt, .. of an nr x nc block whose cell (r, c) is (row(r), col(c)): the loads of
+    // four cells before their stores while there are four, then one by one
+    const auto cells = [&](auto u, int t, int nc, auto row, auto col) {
+        constexpr int U = decltype(u)::value;
+        float x[U], v[U];
+        int rr[U], cc[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int tk = t + k * nt, r = tk / nc;
+            rr[k] = row(r);
+            cc[k] = col(tk - r * nc);
+            const long long o = (long long)rr[k] * pitch + cc[k];
+            x[k] = f0[o];
+            v[k] = f1[o];
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++)
+            for (int i = rr[k] - nx * ((rr[k] + GR) / nx); i < nx + GR; i += nx)
+                for (int j = cc[k] - ny * ((cc[k] + GC) / ny); j < ny + GC; j += ny)
+                    if (i != rr[k] || j != cc[k]) {
+                        f0[(long long)i * pitch + j] = x[k];
+                        f1[(long long)i * pitch + j] = v[k];
+                    }
+    };
+    const auto block = [&](int nr, int nc, auto row, auto col) {
+        int t = t0;
+        for (; t + 3 * nt < nr * nc; t += 4 * nt) cells(std::integral_constant<int, 4>(), t, nc, row, col);
+        for (; t < nr * nc; t += nt) cells(std::integral_constant<int, 1>(), t, nc, row, col);
+    };
+    // the two bands of columns, all rows
+    const int wa = max(0, min(hi, GC) - lo), b0 = max(max(lo, ny - GC), lo + wa), wb = max(0, hi - b0), wc = wa + wb;
+    if (wc > 0) block(i_e - i_s, wc, [&](int r) { return i_s + r; }, [&](int q) { return q < wa ? lo + q : b0 + q - wa; });
+    // the two bands of rows, the columns between
+    const int na = max(0, min(i_e, GR) - i_s), r0 = max(max(i_s, nx - GR), i_s + na), nb = max(0, i_e - r0);
+    if (hi - lo > wc)
+        block(na + nb, hi - lo - wc, [&](int r) { return r < na ? i_s + r : r0 + r - na; }, [&](int q) { return lo + wa + q; });
+}
+
+// A pass over a periodic scene in the ghost layout: every tile is inner, reads its wrapped halo as
+// ordinary neighbours and writes the ghosts of its cells.  A kernel of its own, so that the strips
+// of k_step_skew keep their constants.  Periodic grids took single updates before, at DRAM's rate:
+// 3840x2160, table, 31.3 to 7.5 us an update (1105 Gcell/s); 1277x717 7.0 to 2.6; 256x192, where a launch
+// bounds the update, 4.9 to 1.8.
+template <int COEF, int P, int PL>
+__global__ void __launch_bounds__(32 * P, skew_min_blocks(P))
+    k_step_wrap(const __grid_constant__ DevParams p, const __grid_constant__ TbArgs a, const int4 *__restrict__ tasks, int K)
+{
+    extern __shared__ float4 skew_smem[];
+    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
+    const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int H = (K + 3) & ~3, step = 128 - 2 * H;
+    const int4 t = tasks[blockIdx.x];
+    const int lo = t.x * step, hi = min(lo + step, p.ny);
+    pdl_wait();
+    pdl_trigger();
+    skew_strip<COEF, PL, P, false, false>(p, a, K, t.y, t.z, lo - H + 4 * lane, lane, w, reinterpret_cast<float *>(skew_smem), lo,
+                                          hi, -GR, p.nx + GR, -GC, p.ny + GC);
+    __syncthreads();  // the last warp's rows
+    skew_images(a.phi_out, a.psi_out, p.nx, p.ny, p.pitch, t.y, t.z, lo, hi, threadIdx.x, 32 * P);
+}
+
 static bool skew_shape_ok(const DevParams &p, int K, int S)
 {
     return K >= 2 && K <= WG_SKEW_MAX_K && S >= 8 && S <= 4096 && p.ny >= 8 && p.nx >= 2;
@@ -857,52 +929,54 @@ static int sm_count()
     return n;
 }
 
-template <int COEF, int P, int PL>
+template <int COEF, int P, int PL, bool WRAP>
 static int skew_capacity()
 {
+    const auto kernel = WRAP ? k_step_wrap<COEF, P, PL> : k_step_skew<COEF, P, PL>;
     constexpr size_t smem = SkewShm<COEF, PL, P>::BYTES;
     static int per_sm = 0;
     if (!per_sm) {
-        cudaFuncSetAttribute(k_step_skew<COEF, P, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int nb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step_skew<COEF, P, PL>, 32 * P, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, 32 * P, smem);
         per_sm = nb > 0 ? nb : 1;
     }
     return per_sm * sm_count();
 }
 
 template <int COEF, int P, int PL>
-static int skew_launch(const DevParams &p, const TbArgs *a, int K, const int4 *tasks, int ntasks, cudaStream_t st)
+static int skew_launch(const DevParams &p, const TbArgs *a, int K, const int4 *tasks, int ntasks, cudaStream_t st, bool wrap)
 {
-    const int cap = skew_capacity<COEF, P, PL>();  // sets the shared-memory attribute once
+    // the capacity sets the shared-memory attribute once
+    const int cap = wrap ? skew_capacity<COEF, P, PL, true>() : skew_capacity<COEF, P, PL, false>();
     if (a)
-        launch_pdl(k_step_skew<COEF, P, PL>, dim3((unsigned)ntasks), dim3(32 * P), SkewShm<COEF, PL, P>::BYTES, st, p, *a, tasks,
-                   K);
+        launch_pdl(wrap ? k_step_wrap<COEF, P, PL> : k_step_skew<COEF, P, PL>, dim3((unsigned)ntasks), dim3(32 * P),
+                   SkewShm<COEF, PL, P>::BYTES, st, p, *a, tasks, K);
     return cap;
 }
 
 template <int COEF, int PL>
-static int skew_dispatch(const DevParams &p, const TbArgs *a, int K, const int4 *tasks, int ntasks, cudaStream_t st)
+static int skew_dispatch(const DevParams &p, const TbArgs *a, int K, const int4 *tasks, int ntasks, cudaStream_t st, bool wrap)
 {
     switch ((K + 1) / 2) {
-    case 1: return skew_launch<COEF, 1, PL>(p, a, K, tasks, ntasks, st);
-    case 2: return skew_launch<COEF, 2, PL>(p, a, K, tasks, ntasks, st);
-    default: return skew_launch<COEF, 3, PL>(p, a, K, tasks, ntasks, st);
+    case 1: return skew_launch<COEF, 1, PL>(p, a, K, tasks, ntasks, st, wrap);
+    case 2: return skew_launch<COEF, 2, PL>(p, a, K, tasks, ntasks, st, wrap);
+    default: return skew_launch<COEF, 3, PL>(p, a, K, tasks, ntasks, st, wrap);
     }
 }
 
 // Launches a pass (a != nullptr) and returns the number of resident teams.
-static int skew_call(const DevParams &p, const TbArgs *a, int coef, int K, const int4 *tasks, int ntasks, cudaStream_t st)
+static int skew_call(const DevParams &p, const TbArgs *a, int coef, int K, const int4 *tasks, int ntasks, cudaStream_t st, bool wrap)
 {
     const int pl = skew_form(p.twospeeds, p.floor_clamp, p.kappa);
     if (coef == WG_COEF_TABLE) {
-        if (pl == PL_ALL) return skew_dispatch<WG_COEF_TABLE, PL_ALL>(p, a, K, tasks, ntasks, st);
-        if (pl == PL_MASKED) return skew_dispatch<WG_COEF_TABLE, PL_MASKED>(p, a, K, tasks, ntasks, st);
-        return skew_dispatch<WG_COEF_TABLE, PL_GEN>(p, a, K, tasks, ntasks, st);
+        if (pl == PL_ALL) return skew_dispatch<WG_COEF_TABLE, PL_ALL>(p, a, K, tasks, ntasks, st, wrap);
+        if (pl == PL_MASKED) return skew_dispatch<WG_COEF_TABLE, PL_MASKED>(p, a, K, tasks, ntasks, st, wrap);
+        return skew_dispatch<WG_COEF_TABLE, PL_GEN>(p, a, K, tasks, ntasks, st, wrap);
     }
-    if (pl == PL_ALL) return skew_dispatch<WG_COEF_MASK, PL_ALL>(p, a, K, tasks, ntasks, st);
-    if (pl == PL_MASKED) return skew_dispatch<WG_COEF_MASK, PL_MASKED>(p, a, K, tasks, ntasks, st);
-    return skew_dispatch<WG_COEF_MASK, PL_GEN>(p, a, K, tasks, ntasks, st);
+    if (pl == PL_ALL) return skew_dispatch<WG_COEF_MASK, PL_ALL>(p, a, K, tasks, ntasks, st, wrap);
+    if (pl == PL_MASKED) return skew_dispatch<WG_COEF_MASK, PL_MASKED>(p, a, K, tasks, ntasks, st, wrap);
+    return skew_dispatch<WG_COEF_MASK, PL_GEN>(p, a, K, tasks, ntasks, st, wrap);
 }
 
 // Task list of a skewed pass.  Every column tile is cut into row chunks; a chunk costs its
@@ -990,14 +1064,27 @@ static std::vector<int4> skew_plan(const DevParams &p, int K, int min_rows, int 
     return out;
 }
 
+// The same for a periodic scene: all strips cost the same, so every tile is cut into equal chunks of
+// at least min_rows rows, as many as fill the resident teams once.
+static std::vector<int4> wrap_plan(const DevParams &p, int K, int min_rows, int cap)
+{
+    const int step = 128 - 2 * ((K + 3) & ~3), tiles = (p.ny + step - 1) / step;
+    const int n = std::max(1, std::min(p.nx / std::max(min_rows, 1), cap / tiles));
+    std::vector<int4> out;
+    for (int q = 0; q < n; q++)
+        for (int tj = 0; tj < tiles; tj++)
+            out.push_back(make_int4(tj, (int)((long long)q * p.nx / n), (int)((long long)(q + 1) * p.nx / n), 0));
+    return out;
+}
+
 // Task list of (depth K, minimum rows L) for this scene, built once and kept on the device.
 static wg_status skew_tasks(wg_scene *s, int K, int L, const int4 **tasks, int *ntasks)
 {
     if (K < 0 || K > WG_SKEW_MAX_K) { set_error("skewed depth %d outside 0..%d", K, WG_SKEW_MAX_K); return WG_ERR_INVALID; }
     SkewPlanCache &c = s->skew[K];
     if (!c.dev || c.min_rows != L) {
-        const int cap = skew_call(s->dp, nullptr, s->coef, K, nullptr, 0, s->st);
-        const std::vector<int4> v = skew_plan(s->dp, K, L, cap);
+        const int cap = skew_call(s->dp, nullptr, s->coef, K, nullptr, 0, s->st, s->wrap);
+        const std::vector<int4> v = s->wrap ? wrap_plan(s->dp, K, L, cap) : skew_plan(s->dp, K, L, cap);
         if (c.dev) cudaFree(c.dev);
         c.dev = nullptr;
         WG_CUDA(cudaMalloc(&c.dev, v.size() * sizeof(int4)));
@@ -1026,55 +1113,6 @@ static wg_status skew_tasks(wg_scene *s, int K, int L, const int4 **tasks, int *
 // 512 a side, absorbing: 333 to 285 us for 10 updates).
 // ---------------------------------------------------------------------------
 static_assert(sizeof(DevParams) % 4 == 0, "DevParams is copied as 32-bit words");
-
-// The ghost cells that mirror the rows [i_s, i_e) and columns [lo, hi) of a wrapped scene's new
-// fields, by the team that stored them: a cell within BATCH_GHOST_COLS of the left or right edge or
-// BATCH_GHOST_ROWS of the top or bottom one goes to every place of the extended grid that wraps to
-// it.  (The last group of four columns may reach past ny-1; the cells it stores there are the
-// same values.)  A kernel before each pass did this over the whole batch, 22 us with 48 scenes, and
-// kept passes from overlapping: 48 scenes of 256 to 960 a side, half of them periodic, 10 updates:
-// 224 to 195 us.
-__device__ __noinline__ void skew_images(float *f0, float *f1, int nx, int ny, int pitch, int i_s, int i_e, int lo, int hi,
-                                         int t0, int nt)
-{
-    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
-    // cells t0, t0 + nt, .. of an nr x nc block whose cell (r, c) is (row(r), col(c)): the loads of
-    // four cells before their stores while there are four, then one by one
-    const auto cells = [&](auto u, int t, int nc, auto row, auto col) {
-        constexpr int U = decltype(u)::value;
-        float x[U], v[U];
-        int rr[U], cc[U];
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            const int tk = t + k * nt, r = tk / nc;
-            rr[k] = row(r);
-            cc[k] = col(tk - r * nc);
-            const long long o = (long long)rr[k] * pitch + cc[k];
-            x[k] = f0[o];
-            v[k] = f1[o];
-        }
-#pragma unroll
-        for (int k = 0; k < U; k++)
-            for (int i = rr[k] - nx * ((rr[k] + GR) / nx); i < nx + GR; i += nx)
-                for (int j = cc[k] - ny * ((cc[k] + GC) / ny); j < ny + GC; j += ny)
-                    if (i != rr[k] || j != cc[k]) {
-                        f0[(long long)i * pitch + j] = x[k];
-                        f1[(long long)i * pitch + j] = v[k];
-                    }
-    };
-    const auto block = [&](int nr, int nc, auto row, auto col) {
-        int t = t0;
-        for (; t + 3 * nt < nr * nc; t += 4 * nt) cells(std::integral_constant<int, 4>(), t, nc, row, col);
-        for (; t < nr * nc; t += nt) cells(std::integral_constant<int, 1>(), t, nc, row, col);
-    };
-    // the two bands of columns, all rows
-    const int wa = max(0, min(hi, GC) - lo), b0 = max(max(lo, ny - GC), lo + wa), wb = max(0, hi - b0), wc = wa + wb;
-    if (wc > 0) block(i_e - i_s, wc, [&](int r) { return i_s + r; }, [&](int q) { return q < wa ? lo + q : b0 + q - wa; });
-    // the two bands of rows, the columns between
-    const int na = max(0, min(i_e, GR) - i_s), r0 = max(max(i_s, nx - GR), i_s + na), nb = max(0, i_e - r0);
-    if (hi - lo > wc)
-        block(na + nb, hi - lo - wc, [&](int r) { return r < na ? i_s + r : r0 + r - na; }, [&](int q) { return lo + wa + q; });
-}
 
 template <int P, int PL>
 __global__ void __launch_bounds__(32 * P, P == 1 ? 16 : skew_min_blocks(P))
@@ -1330,23 +1368,27 @@ static bool tb_depth_ok(int k) { return k >= 2 && k <= 8; }
 
 bool tb_supported(const wg_scene *s)
 {
-    return s->prec == WG_FP32 && (s->prm.b_cond == WG_BC_DIRICHLET || s->prm.b_cond == WG_BC_ABSORBING) &&
+    return s->prec == WG_FP32 && (s->prm.b_cond == WG_BC_DIRICHLET || s->prm.b_cond == WG_BC_ABSORBING || s->wrap) &&
            s->nrec == 0 && !s->has_ghosts && (s->coef == WG_COEF_MASK || s->tg == nullptr);
 }
 
 static wg_status ensure_tb_buffers(wg_scene *s)
 {
-    const size_t fb = (size_t)s->prm.nx * s->pitch * s->esz;
     for (int k = 0; k < 2; k++)
-        if (!s->g[k]) {
-            WG_CUDA(cudaMalloc(&s->g[k], fb));
-            WG_CUDA(cudaMemsetAsync(s->g[k], 0, fb, s->st));
-        }
+        if (!s->g[k])
+            if (wg_status st = scene_alloc_field(s, &s->g[k])) return st;
     return WG_OK;
 }
 
 wg_status tb_prepare(wg_scene *s, int n)
 {
+    if (s->wrap && !s->mask_ghosts_ok) {
+        launch_act_ghosts(s->act, s->dp.wpitch, s->prm.nx, s->prm.ny, s->st);
+        if (s->tcc) launch_grid_ghosts((float *)s->tcc, nullptr, s->prm.nx, s->prm.ny, s->pitch, s->st);
+        s->launches += s->tcc ? 2 : 1;
+        WG_CUDA(cudaGetLastError());
+        s->mask_ghosts_ok = true;
+    }
     if (!s->prm.oscillate_left && !s->prm.src_on) return WG_OK;
     const size_t need = (size_t)n * (s->prm.oscillate_left ? s->prm.ny : 1);
     if (need > s->bv_cap) {
@@ -1413,7 +1455,12 @@ wg_status tb_pass<float>(wg_scene *s, int k)
         const int4 *tasks = nullptr;
         int ntasks = 0;
         if ((st = skew_tasks(s, k, L, &tasks, &ntasks))) return st;
-        skew_call(s->dp, &a, s->coef, k, tasks, ntasks, s->st);
+        if (s->wrap && !s->ghosts_ok) {
+            launch_grid_ghosts((float *)s->f[s->cur], (float *)s->f[1 - s->cur], s->prm.nx, s->prm.ny, s->pitch, s->st);
+            s->launches++;
+        }
+        skew_call(s->dp, &a, s->coef, k, tasks, ntasks, s->st, s->wrap);
+        s->ghosts_ok = s->wrap;
     } else if (clear_error(), !launch_tb(s, a, k, L, W)) {
         if (wg_last_error()[0] == 0) set_error("unsupported temporal block (depth %d, tile %d x %d)", k, L, W);
         return WG_ERR_INVALID;
@@ -1473,14 +1520,14 @@ void autotune_scene(wg_scene *s)
         }
     }
     // save the state, time the candidates, restore the state
-    const size_t fb = (size_t)s->prm.nx * s->pitch * s->esz;
+    const size_t fb = s->field_bytes;
     void *save[2] = {nullptr, nullptr};
     bool ok = ensure_tb_buffers(s) == WG_OK;
     for (int k = 0; k < 2 && ok; k++) ok = cudaMalloc(&save[k], fb) == cudaSuccess;
     int best_k = 1, best_l = 0, best_w = 0;
     if (ok) {
-        cudaMemcpyAsync(save[0], s->f[0], fb, cudaMemcpyDeviceToDevice, s->st);
-        cudaMemcpyAsync(save[1], s->f[1], fb, cudaMemcpyDeviceToDevice, s->st);
+        cudaMemcpyAsync(save[0], scene_field_base(s, s->f[0]), fb, cudaMemcpyDeviceToDevice, s->st);
+        cudaMemcpyAsync(save[1], scene_field_base(s, s->f[1]), fb, cudaMemcpyDeviceToDevice, s->st);
         const long long t_save = s->time;
         const int cur_save = s->cur;
         cudaEvent_t e0, e1;
@@ -1523,10 +1570,11 @@ void autotune_scene(wg_scene *s)
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         s->cur = cur_save;
-        cudaMemcpyAsync(s->f[0], save[0], fb, cudaMemcpyDeviceToDevice, s->st);
-        cudaMemcpyAsync(s->f[1], save[1], fb, cudaMemcpyDeviceToDevice, s->st);
+        cudaMemcpyAsync(scene_field_base(s, s->f[0]), save[0], fb, cudaMemcpyDeviceToDevice, s->st);
+        cudaMemcpyAsync(scene_field_base(s, s->f[1]), save[1], fb, cudaMemcpyDeviceToDevice, s->st);
         cudaStreamSynchronize(s->st);
         s->time = t_save;
+        s->ghosts_ok = false;
     }
     for (void *p : save)
         if (p) cudaFree(p);
