@@ -439,7 +439,9 @@ struct SkewShm {
     static constexpr int IN = 0, HAND = IN + SK_IN * 512, TCC = HAND + (P - 1) * 1024,
                          ACT = TCC + (COEF == WG_COEF_TABLE ? NT * 256 : 0), TCE = ACT + (NEED_ACT ? NT * 64 : 0),
                          SIZE = TCE + (COEF == WG_COEF_TABLE ? NT * 64 : 0);
-    static constexpr size_t BYTES = SIZE * sizeof(float);
+    // single grids with OSCILLATE_LEFT: row 0's values at the tile's columns, per level
+    static constexpr int OSC = SIZE;
+    static constexpr size_t BYTES = SIZE * sizeof(float), OSC_BYTES = 2 * P * 128 * sizeof(float);
 };
 
 // What an edge strip knows.  EDGE of a step: 0 inner; 1 the tile holds column 0 or ny-1 (mirror
@@ -450,6 +452,7 @@ struct SkewEdge {
     bool left, right;        // the tile holds column 0, column ny-1 (warp-uniform)
     bool my_left, my_right;  // this lane holds it
     bool src, absorb;        // the lane holds the point source's column; B_COND is absorbing
+    const float *osc;        // OSCILLATE_LEFT's values at the lane's columns, 128 floats a level
 };
 
 // Cell k's absorbing rule along j on the lanes of `mine`; d = x - (its inward neighbour).
@@ -481,7 +484,7 @@ __device__ __forceinline__ void skew_row_edge(const DevParams &p, const TbArgs &
     const float x = el<k>(c), y = el<k>(cv);
     XV n;
     if (r == 0 && left_bc(p, gj)) {
-        n = set32(x, INL ? osc_inl(p, a.t0 + lv, gj) : a.osc[(size_t)(lv - 1) * p.ny + gj]);
+        n = set32(x, INL ? osc_inl(p, a.t0 + lv, gj) : ed.osc[(lv - 1) * 128 + k]);
     } else if (ed.absorb && (p.twospeeds || ac)) {
         const float d = r == 0 ? -el<k>(dn) : el<k>(D);
         const float tcv = (COEF == WG_COEF_TABLE) ? (a.tc ? a.tc[(size_t)r * p.pitch + gj] : 0.f)
@@ -498,13 +501,14 @@ __device__ __forceinline__ void skew_row_edge(const DevParams &p, const TbArgs &
 
 // Cell k: a corner of OSCILLATE_LEFT, then the point source.
 template <bool INL, int k>
-__device__ __forceinline__ void skew_corner_src(const DevParams &p, const TbArgs &a, int lv, int gj0, const f2 (&c)[2],
+__device__ __forceinline__ void skew_corner_src(const DevParams &p, const TbArgs &a, const SkewEdge &ed, int lv, int gj0,
+                                                const f2 (&c)[2],
                                                 unsigned act, bool corner, bool src, f2 (&ox)[2], f2 (&ov)[2])
 {
     const int gj = gj0 + k;
     XV n = XV{el<k>(ox), el<k>(ov)};
     if (corner && gj < p.ny && (gj == 0 || (p.corner2_on && gj == p.nx - 1))) {
-        n = set32(el<k>(c), INL ? osc_inl(p, a.t0 + lv, gj) : a.osc[(size_t)(lv - 1) * p.ny + gj]);
+        n = set32(el<k>(c), INL ? osc_inl(p, a.t0 + lv, gj) : ed.osc[(lv - 1) * 128 + k]);
         if (p.floor_clamp && ((act >> k) & 1u)) n = clamp32(el<k>(c), n, a.vmax);
     }
     if (src && gj == p.src_j) n = source32(n, INL ? src_inl(p, a.t0 + lv) : a.src[lv - 1]);
@@ -571,10 +575,10 @@ __device__ __forceinline__ void skew_level(const DevParams &p, const TbArgs &a, 
     if (EDGE == 2) {
         const bool corner = r == 0 && p.osc_left && !p.beam, src = ed.src && r == p.src_i;
         if (corner || src) {
-            skew_corner_src<INL, 0>(p, a, lv, gj0, c, act, corner, src, ox, ov);
-            skew_corner_src<INL, 1>(p, a, lv, gj0, c, act, corner, src, ox, ov);
-            skew_corner_src<INL, 2>(p, a, lv, gj0, c, act, corner, src, ox, ov);
-            skew_corner_src<INL, 3>(p, a, lv, gj0, c, act, corner, src, ox, ov);
+            skew_corner_src<INL, 0>(p, a, ed, lv, gj0, c, act, corner, src, ox, ov);
+            skew_corner_src<INL, 1>(p, a, ed, lv, gj0, c, act, corner, src, ox, ov);
+            skew_corner_src<INL, 2>(p, a, ed, lv, gj0, c, act, corner, src, ox, ov);
+            skew_corner_src<INL, 3>(p, a, ed, lv, gj0, c, act, corner, src, ox, ov);
         }
     }
     D[0] = dn[0];
@@ -630,7 +634,7 @@ __device__ __forceinline__ void skew_strip(const DevParams &p, const TbArgs &a, 
     const bool last = w == P - 1;
     const bool col_ok = gj0 >= clo && gj0 < chi;
     const bool core = gj0 >= lo && gj0 < hi && gj0 >= 0 && gj0 < p.ny;
-    SkewEdge ed = {-1, -1, -1, -1, -1, 0, false, false, false, false, false, false};
+    SkewEdge ed = {-1, -1, -1, -1, -1, 0, false, false, false, false, false, false, nullptr};
     if (EDGE) {
         const int cr = p.ny - 1 - gj0;  // column ny-1 within the lane's group when 0..3
         const int t0 = gj0 - 4 * lane;
@@ -652,6 +656,21 @@ __device__ __forceinline__ void skew_strip(const DevParams &p, const TbArgs &a, 
     const float *const my1 = shm + lane;
     const unsigned base16 = (unsigned)__cvta_generic_to_shared(my4), base4 = (unsigned)__cvta_generic_to_shared(my1);
     const long long pitch = p.pitch;
+    if (EDGE && !INL) {
+        // Each warp fetches row 0's values of its two levels ahead.  Read where they are used, their
+        // latencies, one after the other in every level, made the first rows' strips last longest
+        // (1277x717, 50 updates a call: 4.21 to 3.79 us an update).
+        ed.osc = my4 + SM::OSC;
+        if (p.osc_left && i_s < K) {
+#pragma unroll 1
+            for (int lv = 2 * w + 1; lv <= min(2 * w + 2, K); lv++)
+                for (int k = 0; k < 4; k++)
+                    if (gj0 + k >= 0 && gj0 + k < p.ny)
+                        cp_async4s(base16 + 4 * (SM::OSC + (lv - 1) * 128 + k), a.osc + ((size_t)(lv - 1) * p.ny + gj0 + k));
+            cp_async_commit();
+            if (w > 0) cp_async_wait<0>();  // (warp 0: with its first rows)
+        }
+    }
 
     // warp 0: copies of the next two rows (row m_in and the one after it) into input slot si and
     // lagged slot ti (in bytes from the rings' start), while the strip has more rows
@@ -936,7 +955,7 @@ static int skew_capacity()
     constexpr size_t smem = SkewShm<COEF, PL, P>::BYTES;
     static int per_sm = 0;
     if (!per_sm) {
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + SkewShm<COEF, PL, P>::OSC_BYTES));
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, 32 * P, smem);
         per_sm = nb > 0 ? nb : 1;
@@ -951,7 +970,7 @@ static int skew_launch(const DevParams &p, const TbArgs *a, int K, const int4 *t
     const int cap = wrap ? skew_capacity<COEF, P, PL, true>() : skew_capacity<COEF, P, PL, false>();
     if (a)
         launch_pdl(wrap ? k_step_wrap<COEF, P, PL> : k_step_skew<COEF, P, PL>, dim3((unsigned)ntasks), dim3(32 * P),
-                   SkewShm<COEF, PL, P>::BYTES, st, p, *a, tasks, K);
+                   SkewShm<COEF, PL, P>::BYTES + (p.osc_left ? SkewShm<COEF, PL, P>::OSC_BYTES : 0), st, p, *a, tasks, K);
     return cap;
 }
 
