@@ -766,9 +766,8 @@ static wg_status di_energy_all(double **phi, double **psi, int16_t **xy, int ile
     wg_status s = di_energy_fields(phi, psi, xy, &a, &b);
     if (s) return s;
     launch_energy<double>(g_di.dp, g_di.buf[a], g_di.buf[b], g_di.xy, nullptr, g_di.ebot, g_di.etop, ileft, iright,
-                          g_di.eout, g_di.st);
+                          g_di.hout, g_di.prm.nx, nullptr, nullptr, g_di.st);
     WG_CUDA(cudaGetLastError());
-    WG_CUDA(cudaMemcpyAsync(g_di.hout, g_di.eout, sizeof(double) * (g_di.prm.nx + 7), cudaMemcpyDeviceToHost, g_di.st));
     WG_CUDA(cudaStreamSynchronize(g_di.st));
     return WG_OK;
 }

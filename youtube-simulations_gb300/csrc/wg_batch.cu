@@ -833,7 +833,7 @@ wg_status wg_batch_destroy(wg_batch *b)
     batch_drop_graphs(b);
     for (auto &h : b->slots) {
         if (!h.used) continue;
-        void *ptrs[] = {h.mem[0], h.mem[1], h.mem[2], h.mem[3], h.act_mem, h.nz_mem, h.ebot, h.etop, h.eout};
+        void *ptrs[] = {h.mem[0], h.mem[1], h.mem[2], h.mem[3], h.act_mem, h.nz_mem, h.ebot, h.etop};
         for (void *p : ptrs) if (p) cudaFree(p);
     }
     for (auto &kv : b->lists) if (kv.second.dev) cudaFree(kv.second.dev);
@@ -888,11 +888,10 @@ wg_status wg_batch_add(wg_batch *b, const wg_params *p, const double *phi, const
     h.nz = h.nz_mem ? h.nz_mem + L.mask_off : nullptr;
     if (e == cudaSuccess) e = cudaMallocAsync((void **)&h.ebot, p->nx * sizeof(double2), b->st);
     if (e == cudaSuccess) e = cudaMallocAsync((void **)&h.etop, p->nx * sizeof(double2), b->st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void **)&h.eout, (p->nx + 8) * sizeof(double), b->st);
     void *stage = nullptr;
     if (e == cudaSuccess) e = cudaMallocAsync(&stage, 2 * n * sizeof(double), b->st);
     if (e != cudaSuccess) {
-        void *ptrs[] = {h.mem[0], h.mem[1], h.mem[2], h.mem[3], h.act_mem, h.nz_mem, h.ebot, h.etop, h.eout, stage};
+        void *ptrs[] = {h.mem[0], h.mem[1], h.mem[2], h.mem[3], h.act_mem, h.nz_mem, h.ebot, h.etop, stage};
         for (void *q : ptrs) if (q) cudaFreeAsync(q, b->st);
         h = BatchSlotHost();
         return cuda_fail(e, "wg_batch_add");
@@ -950,7 +949,7 @@ wg_status wg_batch_remove(wg_batch *b, int32_t slot)
     BatchSlotHost &h = b->slots[slot];
     h.used = false;
     wg_status st = batch_refresh_table(b);  // the kernels stop seeing the slot first
-    void *ptrs[] = {h.mem[0], h.mem[1], h.mem[2], h.mem[3], h.act_mem, h.nz_mem, h.ebot, h.etop, h.eout};
+    void *ptrs[] = {h.mem[0], h.mem[1], h.mem[2], h.mem[3], h.act_mem, h.nz_mem, h.ebot, h.etop};
     for (void *p : ptrs) if (p) WG_CUDA(cudaFreeAsync(p, b->st));
     h = BatchSlotHost();
     return st;
@@ -1067,12 +1066,13 @@ wg_status wg_batch_energy(wg_batch *b, int32_t slot, double *total)
     // FP32: phi and the velocity of the current pair; FP64: phi and psi of pair 0
     const void *phi = h.f[2 * d.pair + d.cur], *psi = h.f[2 * d.pair + 1 - d.cur];
     if (b->prec == WG_FP32)
-        launch_energy<float>(h.dp, (const float *)phi, (const float *)psi, nullptr, h.nz, h.ebot, h.etop, 0, 0, h.eout, b->st);
+        launch_energy<float>(h.dp, (const float *)phi, (const float *)psi, nullptr, h.nz, h.ebot, h.etop, 0, 0, b->h_out, 0,
+                             nullptr, nullptr, b->st);
     else
-        launch_energy<double>(h.dp, (const double *)phi, (const double *)psi, nullptr, h.nz, h.ebot, h.etop, 0, 0, h.eout, b->st);
+        launch_energy<double>(h.dp, (const double *)phi, (const double *)psi, nullptr, h.nz, h.ebot, h.etop, 0, 0, b->h_out, 0,
+                             nullptr, nullptr, b->st);
     b->launches += 2;
     WG_CUDA(cudaGetLastError());
-    WG_CUDA(cudaMemcpyAsync(b->h_out, h.eout, sizeof(double), cudaMemcpyDeviceToHost, b->st));
     WG_CUDA(cudaStreamSynchronize(b->st));
     *total = b->h_out[0];
     return WG_OK;

@@ -97,7 +97,6 @@ struct BatchSlotHost {
     uint32_t *act_mem = nullptr, *nz_mem = nullptr;
     uint32_t *act = nullptr, *nz = nullptr;
     double2 *ebot = nullptr, *etop = nullptr;
-    double *eout = nullptr;
     size_t bytes = 0;
     bool skew = false;      // FP32 scene whose boundaries the skewed passes cover
     bool wrap = false;      // periodic, in the ghost layout

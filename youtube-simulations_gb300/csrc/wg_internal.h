@@ -84,7 +84,7 @@ template <class T> void launch_neumann_fast(const DevParams &p, const T *phi, T 
                                             const double2 *w, int n, cudaStream_t st);
 template <class T> void launch_energy(const DevParams &p, const T *phi, const T *psi, const int16_t *xy,
                                       const uint32_t *nz, double2 *bot, double2 *top, int ileft, int iright,
-                                      double *out, cudaStream_t st);
+                                      double *out, int ncols, const int *flag, int *hflag, cudaStream_t st);
 template <class T> void launch_count_nonfinite(int nx, int ny, int pitch, const T *a, unsigned long long *count,
                                                cudaStream_t st);
 void launch_pack_mask(int nx, int ny, int wpitch, const int16_t *xy, uint32_t *act, uint32_t *nz, cudaStream_t st);

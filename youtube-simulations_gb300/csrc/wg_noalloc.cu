@@ -119,7 +119,7 @@ extern "C" wg_status wg_compute_energy_device_noalloc(const wg_params *p, const 
     if ((st = scratch_in_current_context(&scratch))) return st;
     const DevParams dp = make_dev_params(*p, pitch);
     launch_energy<double>(dp, phi, psi, xy, nullptr, scratch, scratch + WG_NOALLOC_MAX_NX, ileft, iright, out,
-                          (cudaStream_t)stream);
+                          p->nx, nullptr, nullptr, (cudaStream_t)stream);
     WG_CUDA(cudaGetLastError());
     return WG_OK;
 }

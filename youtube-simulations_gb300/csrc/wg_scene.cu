@@ -90,7 +90,7 @@ size_t scene_device_bytes(const wg_params &p, int prec, int coef)
         if (p.b_cond == WG_BC_ABSORBING || p.b_cond == WG_BC_VPER_HABS) b += L.field_bytes;  // tc
     }
     if (prec == WG_FP32) b += 2 * L.field_bytes;        // FP32: the output pair of every update
-    b += (size_t)p.nx * 2 * sizeof(double2) + (p.nx + 8) * sizeof(double) + 64;  // energy scratch
+    b += (size_t)p.nx * 2 * sizeof(double2) + 64;  // energy scratch
     return b;
 }
 
@@ -353,7 +353,6 @@ wg_status wg_scene_create(const wg_params *p, int32_t precision, int32_t coef_mo
     }
     if (e == cudaSuccess) e = cudaMalloc(&s->ebot, p->nx * sizeof(double2));
     if (e == cudaSuccess) e = cudaMalloc(&s->etop, p->nx * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMalloc(&s->eout, (p->nx + 8) * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&s->dcount, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&s->dflag, sizeof(int));
     if (e == cudaSuccess) e = cudaMemsetAsync(s->dflag, 0, sizeof(int), s->st);
@@ -376,7 +375,7 @@ wg_status wg_scene_destroy(wg_scene *s)
     void *fields[] = {s->f[0], s->f[1], s->g[0], s->g[1], s->tcc, s->tc};
     for (void *f : fields) if (f) cudaFree(scene_field_base(s, f));
     for (uint32_t *m : {s->act, s->nz}) if (m) cudaFree(m - s->mask_off);
-    void *dev[] = {s->tg, s->nidx, s->nw, s->ebot, s->etop, s->eout, s->dcount,
+    void *dev[] = {s->tg, s->nidx, s->nw, s->ebot, s->etop, s->dcount,
                    s->dstage, s->rgb, s->lut, s->bv_osc, s->bv_src, s->dflag, s->facc, s->probe_cells, s->probe_buf,
                    s->nrec_dev};
     for (void *d : dev) if (d) cudaFree(d);
@@ -556,19 +555,17 @@ wg_status wg_scene_energy(wg_scene *s, double *total, double *columns, int32_t i
 {
     if (!s) { set_error("NULL scene"); return WG_ERR_INVALID; }
     const void *phi = s->f[s->cur], *psi = s->f[1 - s->cur];
+    // the sums, and the bounded-wait flag in the last slot, go straight to the pinned buffer
+    int *hflag = reinterpret_cast<int *>(s->hout + s->prm.nx + 7);
+    const int ncols = columns ? s->prm.nx : 0;
     if (s->prec == WG_FP32)
         launch_energy<float>(s->dp, (const float *)phi, (const float *)psi, nullptr, s->nz, s->ebot, s->etop, ileft,
-                             iright, s->eout, s->st);
+                             iright, s->hout, ncols, s->dflag, hflag, s->st);
     else
         launch_energy<double>(s->dp, (const double *)phi, (const double *)psi, nullptr, s->nz, s->ebot, s->etop, ileft,
-                              iright, s->eout, s->st);
+                              iright, s->hout, ncols, s->dflag, hflag, s->st);
     s->launches += 2;
     WG_CUDA(cudaGetLastError());
-    const size_t nout = columns ? (size_t)s->prm.nx + 7 : 7;
-    WG_CUDA(cudaMemcpyAsync(s->hout, s->eout, nout * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-    // the bounded-wait flag rides in the last slot of the same pinned buffer: one sync
-    int *hflag = reinterpret_cast<int *>(s->hout + s->prm.nx + 7);
-    WG_CUDA(cudaMemcpyAsync(hflag, s->dflag, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     WG_CUDA(cudaStreamSynchronize(s->st));
     if (*hflag) {
         WG_CUDA(cudaMemsetAsync(s->dflag, 0, sizeof(int), s->st));

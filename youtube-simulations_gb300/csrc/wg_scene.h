@@ -39,7 +39,7 @@ struct wg_scene {
     int nrec_all = 0;
     long long time = 0, launches = 0;
     double2 *ebot = nullptr, *etop = nullptr;
-    double *eout = nullptr, *hout = nullptr;
+    double *hout = nullptr;
     unsigned long long *dcount = nullptr;
     int *dflag = nullptr;          // set by a kernel whose bounded wait gave up
     void *dstage = nullptr;
