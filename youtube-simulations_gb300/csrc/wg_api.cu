@@ -164,6 +164,7 @@ struct DropIn {
     const void *rec_key = nullptr;
     int rec_key_n = -1;
     bool statics_valid = false, energy_statics_valid = false;
+    bool rows_pending = false;  // kernels of the current call still use the caller's rows
     void *hstage = nullptr;
     size_t hstage_bytes = 0;
     double2 *ebot = nullptr, *etop = nullptr;
@@ -199,6 +200,28 @@ static wg_status di_stage(size_t bytes)
     g_di.hstage_bytes = bytes;
     return WG_OK;
 }
+
+// Waits for the kernels of this call that read or write the caller's rows in place.  A call
+// waits once, for all of its rows: strict evolve_wave copies ten arrays, and waiting after each
+// left the host link idle in between (1280x720: 542 to 472 us a call).
+static wg_status di_rows_wait()
+{
+    if (!g_di.rows_pending) return WG_OK;
+    g_di.rows_pending = false;
+    WG_CUDA(cudaStreamSynchronize(g_di.st));
+    return WG_OK;
+}
+// The lock of a drop-in call; a call that fails half way still waits before it returns.
+struct DiLock {
+    std::lock_guard<std::mutex> lk{g_di_mu};
+    ~DiLock()
+    {
+        if (g_di.rows_pending) {
+            g_di.rows_pending = false;
+            cudaStreamSynchronize(g_di.st);
+        }
+    }
+};
 
 // Rows read and written in place by the device: one block per row, 16-byte accesses where
 // the row and its byte count allow (a pitched row starts on 512 bytes), the padding zeroed.
@@ -295,11 +318,11 @@ static wg_status di_upload_rows(E **rows, E *dev)
     for (int i = 0; i < nx; i++)
         if (!rows[i]) { set_error("row %d is NULL", i); return WG_ERR_INVALID; }
     if (di_in_place()) {
-        // the kernel reads the caller's row table and rows; the call waits for it, so the
-        // rows may change (or go) as soon as it returns
+        // the kernel reads the caller's row table and rows; the call waits for it before it
+        // returns, so the rows may change (or go) then
+        g_di.rows_pending = true;
         k_rows_in<E><<<nx, 256, 0, g_di.st>>>(rows, nx, ny, P, dev);
         WG_CUDA(cudaGetLastError());
-        WG_CUDA(cudaStreamSynchronize(g_di.st));
         return WG_OK;
     }
     WG_CUDA(cudaStreamSynchronize(g_di.st));  // staging may still feed an earlier copy
@@ -314,17 +337,18 @@ static wg_status di_upload_rows(E **rows, E *dev)
     return WG_OK;
 }
 
-static wg_status di_download_rows(double *dev, double **rows)
+// last = false: another download of the same call follows and waits
+static wg_status di_download_rows(double *dev, double **rows, bool last = true)
 {
     const int nx = g_di.prm.nx, ny = g_di.prm.ny, P = g_di.pitch;
     const size_t bytes = (size_t)nx * P * sizeof(double);
     if (di_in_place()) {
         for (int i = 0; i < nx; i++)
             if (!rows[i]) { set_error("row %d is NULL", i); return WG_ERR_INVALID; }
+        g_di.rows_pending = true;
         k_rows_out<<<nx, 256, 0, g_di.st>>>(rows, nx, ny, P, dev);
         WG_CUDA(cudaGetLastError());
-        WG_CUDA(cudaStreamSynchronize(g_di.st));
-        return WG_OK;
+        return last ? di_rows_wait() : WG_OK;
     }
     wg_status s = di_stage(bytes);
     if (s) return s;
@@ -472,7 +496,7 @@ void wg_params_default(wg_params *p, int32_t nx, int32_t ny)
 
 wg_status wg_dropin_configure(const wg_params *p)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     if (!p) { set_error("params is NULL"); return WG_ERR_INVALID; }
     wg_status s = validate_params(*p);
     if (s) return s;
@@ -508,7 +532,7 @@ wg_status wg_dropin_configure(const wg_params *p)
 
 wg_status wg_dropin_set_mode(int32_t mode)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     if (mode != WG_DROPIN_STRICT && mode != WG_DROPIN_RESIDENT) { set_error("unknown mode %d", mode); return WG_ERR_INVALID; }
     g_di.mode = mode;
     for (auto &h : g_di.host_rows) h = nullptr;
@@ -520,7 +544,7 @@ wg_status wg_dropin_set_mode(int32_t mode)
 
 wg_status wg_dropin_set_rows(int32_t rows_mode)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     if (rows_mode != WG_ROWS_AUTO && rows_mode != WG_ROWS_PACKED) {
         set_error("unknown rows mode %d", rows_mode);
         return WG_ERR_INVALID;
@@ -531,18 +555,18 @@ wg_status wg_dropin_set_rows(int32_t rows_mode)
 
 wg_status wg_dropin_sync(void)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s) return s;
     for (int k = 0; k < 3; k++)
-        if (g_di.host_rows[k] && (s = di_download_rows(g_di.buf[k], g_di.host_rows[k]))) return s;
-    return WG_OK;
+        if (g_di.host_rows[k] && (s = di_download_rows(g_di.buf[k], g_di.host_rows[k], false))) return s;
+    return di_rows_wait();
 }
 
 wg_status wg_dropin_add_circular_wave(double init_amp, double factor, double x, double y, double variance,
                                       double wavelength, double **phi, double **psi, int16_t **xy_in)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s) return s;
     if (!phi || !psi || !xy_in) { set_error("NULL argument"); return WG_ERR_INVALID; }
@@ -557,12 +581,12 @@ wg_status wg_dropin_add_circular_wave(double init_amp, double factor, double x, 
     launch_add_circular_wave<double>(pa, g_di.buf[k], nullptr, g_di.xy, nullptr, g_di.st);
     WG_CUDA(cudaGetLastError());
     if (g_di.mode == WG_DROPIN_STRICT) return di_download_rows(g_di.buf[k], phi);
-    return WG_OK;
+    return di_rows_wait();
 }
 
 wg_status wg_dropin_cell(double **phi, int32_t i, int32_t j, double *out)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s) return s;
     if (!phi || !out || i < 0 || j < 0 || i >= g_di.prm.nx || j >= g_di.prm.ny) { set_error("bad arguments"); return WG_ERR_INVALID; }
@@ -582,7 +606,7 @@ wg_status wg_dropin_cell(double **phi, int32_t i, int32_t j, double *out)
 
 wg_status wg_dropin_invalidate(void)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     for (auto &h : g_di.host_rows) h = nullptr;
     g_di.statics_valid = false;
     g_di.energy_statics_valid = false;
@@ -606,7 +630,7 @@ wg_status wg_dropin_set_time(int64_t t)
 wg_status wg_evolve_wave_half(double **phi_in, double **psi_in, double **phi_out, int16_t **xy_in, double **tcc,
                               double **tc, double **tgamma, const wg_neumann_bc *neumann_bc, int32_t n_neumann)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s) return s;
     if (!phi_in || !psi_in || !phi_out) { set_error("field pointer is NULL"); return WG_ERR_INVALID; }
@@ -624,13 +648,13 @@ wg_status wg_evolve_wave_half(double **phi_in, double **psi_in, double **phi_out
     if (f2 && (s = di_upload_rows<double>(phi_out, g_di.buf[c]))) return s;
     if ((s = di_one_update(a, b, c))) return s;
     if (g_di.mode == WG_DROPIN_STRICT) return di_download_rows(g_di.buf[c], phi_out);
-    return WG_OK;
+    return di_rows_wait();
 }
 
 wg_status wg_evolve_wave(double **phi, double **psi, double **tmp, int16_t **xy_in, double **tcc, double **tc,
                          double **tgamma, const wg_neumann_bc *neumann_bc, int32_t n_neumann)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s) return s;
     if (!phi || !psi || !tmp || phi == psi || phi == tmp || psi == tmp) {
@@ -653,11 +677,11 @@ wg_status wg_evolve_wave(double **phi, double **psi, double **tmp, int16_t **xy_
     if ((s = di_one_update(c, a, b))) return s;
     if ((s = di_one_update(b, c, a))) return s;
     if (g_di.mode == WG_DROPIN_STRICT) {
-        if ((s = di_download_rows(g_di.buf[a], phi))) return s;
-        if ((s = di_download_rows(g_di.buf[b], psi))) return s;
+        if ((s = di_download_rows(g_di.buf[a], phi, false))) return s;
+        if ((s = di_download_rows(g_di.buf[b], psi, false))) return s;
         if ((s = di_download_rows(g_di.buf[c], tmp))) return s;
     }
-    return WG_OK;
+    return di_rows_wait();
 }
 
 static wg_status energy_variant_check()
@@ -680,7 +704,7 @@ static wg_status di_energy_update(int in, int prev, int out)
 
 wg_status wg_evolve_wave_half_energy(double **phi_in, double **psi_in, double **phi_out, int16_t **xy_in)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s || (s = energy_variant_check())) return s;
     if (!phi_in || !psi_in || !phi_out || phi_in == phi_out || psi_in == phi_out) {
@@ -696,12 +720,12 @@ wg_status wg_evolve_wave_half_energy(double **phi_in, double **psi_in, double **
     if (f2 && (s = di_upload_rows<double>(phi_out, g_di.buf[c]))) return s;
     if ((s = di_energy_update(a, b, c))) return s;
     if (g_di.mode == WG_DROPIN_STRICT) return di_download_rows(g_di.buf[c], phi_out);
-    return WG_OK;
+    return di_rows_wait();
 }
 
 wg_status wg_evolve_wave_energy(double **phi, double **psi, double **tmp, int16_t **xy_in)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     wg_status s = di_require();
     if (s || (s = energy_variant_check())) return s;
     if (!phi || !psi || !tmp || phi == psi || phi == tmp || psi == tmp) {
@@ -717,11 +741,11 @@ wg_status wg_evolve_wave_energy(double **phi, double **psi, double **tmp, int16_
     if (f2 && (s = di_upload_rows<double>(tmp, g_di.buf[c]))) return s;
     if ((s = di_energy_update(a, b, c)) || (s = di_energy_update(c, a, b)) || (s = di_energy_update(b, c, a))) return s;
     if (g_di.mode == WG_DROPIN_STRICT) {
-        if ((s = di_download_rows(g_di.buf[a], phi)) || (s = di_download_rows(g_di.buf[b], psi)) ||
+        if ((s = di_download_rows(g_di.buf[a], phi, false)) || (s = di_download_rows(g_di.buf[b], psi, false)) ||
             (s = di_download_rows(g_di.buf[c], tmp)))
             return s;
     }
-    return WG_OK;
+    return di_rows_wait();
 }
 
 // energy of the drop-in fields: upload phi/psi (strict) or use the resident copies
@@ -747,7 +771,7 @@ static wg_status di_energy_fields(double **phi, double **psi, int16_t **xy, int 
 
 wg_status wg_compute_energy(double **phi, double **psi, int16_t **xy_in, int32_t i, int32_t j, double *out)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     int a, b;
     wg_status s = di_energy_fields(phi, psi, xy_in, &a, &b);
     if (s) return s;
@@ -755,7 +779,8 @@ wg_status wg_compute_energy(double **phi, double **psi, int16_t **xy_in, int32_t
     launch_cell_energy(g_di.dp, g_di.buf[a], g_di.buf[b], g_di.xy, i, j, g_di.eout, g_di.st);
     WG_CUDA(cudaGetLastError());
     WG_CUDA(cudaMemcpyAsync(g_di.hout, g_di.eout, sizeof(double), cudaMemcpyDeviceToHost, g_di.st));
-    WG_CUDA(cudaStreamSynchronize(g_di.st));
+    g_di.rows_pending = true;
+    if ((s = di_rows_wait())) return s;
     *out = g_di.hout[0];
     return WG_OK;
 }
@@ -768,13 +793,13 @@ static wg_status di_energy_all(double **phi, double **psi, int16_t **xy, int ile
     launch_energy<double>(g_di.dp, g_di.buf[a], g_di.buf[b], g_di.xy, nullptr, g_di.ebot, g_di.etop, ileft, iright,
                           g_di.hout, g_di.prm.nx, nullptr, nullptr, g_di.st);
     WG_CUDA(cudaGetLastError());
-    WG_CUDA(cudaStreamSynchronize(g_di.st));
-    return WG_OK;
+    g_di.rows_pending = true;
+    return di_rows_wait();
 }
 
 wg_status wg_compute_energy_x_all(double **phi, double **psi, int16_t **xy_in, double *out)
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     if (!out) { set_error("out is NULL"); return WG_ERR_INVALID; }
     wg_status s = di_energy_all(phi, psi, xy_in, 0, 0);
     if (s) return s;
@@ -785,7 +810,7 @@ wg_status wg_compute_energy_x_all(double **phi, double **psi, int16_t **xy_in, d
 wg_status wg_compute_energy_tblr(double **phi, double **psi, int16_t **xy_in, int32_t ileft, int32_t iright,
                                  double energies[6])
 {
-    std::lock_guard<std::mutex> lk(g_di_mu);
+    DiLock lk;
     if (!energies) { set_error("energies is NULL"); return WG_ERR_INVALID; }
     wg_status s = di_energy_all(phi, psi, xy_in, ileft, iright);
     if (s) return s;
