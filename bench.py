@@ -910,7 +910,7 @@ def run_probe(args):
     if args.probe in ("batch", "batch64"):
         rng = np.random.default_rng(1000)
         b = W.Batch(P.FP32 if args.probe == "batch" else P.FP64)
-        b.set_skew(0)  # single updates only: the persistent k_batch_step
+        b.set_skew(0)  # single updates only: the persistent k_batch_step32 / k_batch_step64
         for _ in range(64):
             m = scenes.batch_member(rng)
             b.add(m.params, m.phi, m.psi, m.xy)

@@ -372,7 +372,7 @@ wg_status wg_batch_add(wg_batch *b, const wg_params *p, const double *phi, const
 wg_status wg_batch_remove(wg_batch *b, int32_t slot);
 /* Advances every active scene by nsteps updates, the launches of a frame recorded
  * once as a CUDA graph.  Scenes take single updates (one persistent kernel per update
- * over a tile work queue) or, for FP32 scenes with mirror or absorbing boundaries and
+ * over a work queue) or, for FP32 scenes with mirror, absorbing or periodic boundaries and
  * nsteps >= 2, skewed passes of 2..6 updates at the depth of their size class; both
  * give the same fields bit for bit. */
 wg_status wg_batch_step(wg_batch *b, int32_t nsteps);

@@ -7,7 +7,7 @@
 #define WG_SKEW_MAX_K 6  // deepest skewed pass
 
 struct SkewPlanCache {
-    int4 *dev = nullptr;  // (column tile, first row, end row, edge) per warp
+    int4 *dev = nullptr;  // (column tile, first row, end row, edge) per team of warps
     int n = 0, min_rows = 0;
 };
 

@@ -13,8 +13,8 @@
 // The per-cell rules are the reference's (wave_billiard.c:361-590) for the boundary
 // conditions whose stencils stay inside the tile: the mirror "Dirichlet" box edges,
 // absorbing edges, OSCILLATE_LEFT / OSCILLATE_TOPBOT, FLOOR and the point source.
-// Periodic and VPER_HABS boundaries (which read the opposite side of the grid) and
-// Neumann gathers use the single-step kernel.
+// Periodic grids take skewed passes in a ghost layout (k_step_wrap); VPER_HABS boundaries
+// (which read the opposite side of the grid) and Neumann gathers use the single-step kernel.
 #include <algorithm>
 #include <type_traits>
 #include <cmath>
