@@ -33,7 +33,12 @@ __global__ void __launch_bounds__(128, 4) k_step64(const __grid_constant__ DevPa
                                                    int edge_blocks, int strips, int rows, long long time)
 {
     pdl_wait();  // launched by launch_pdl: the previous update has completed
-    pdl_trigger();
+    // The next launch may come from here on where this one leaves most SMs free (fewer blocks than
+    // SMs: 71x88, 4.1 to 3.8 us an update), otherwise after the work: its blocks, resident early, would
+    // crowd the SMs that this one leaves first, and a launch of less than a wave that is bound by
+    // the FP64 pipe would run at their rate (650x2026, an update and an energy: 294 us so, 171 now).
+    const bool few = gridDim.x <= 152;
+    if (few) pdl_trigger();
     if ((int)blockIdx.x < edge_blocks) {  // a thread per boundary-line cell
         const int q = blockIdx.x * 128 + threadIdx.x;
         if (q < edge64_cells(p)) edge64_cell<COEF, EXACT>(p, a, q, time);
@@ -43,6 +48,7 @@ __global__ void __launch_bounds__(128, 4) k_step64(const __grid_constant__ DevPa
     const int chunk = w / strips, base = (w - chunk * strips) * ST_COLS, r0 = 1 + chunk * rows;
     if (r0 >= p.nx - 1) return;  // warp-uniform
     strip64<COEF, EXACT, Z>(p, a, base, r0, min(r0 + rows, p.nx - 1), time);
+    if (!few) pdl_trigger();
 }
 
 template <int COEF, bool EXACT, int Z>
