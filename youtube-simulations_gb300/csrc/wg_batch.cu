@@ -246,8 +246,9 @@ __device__ __forceinline__ void ghost_fill(float *f0, float *f1, int nx, int ny,
             const int g = (int)t - i * 2 * GC;
             j = g < GC ? g - GC : ny + g - GC;
         } else {  // the ghost rows, over the extended width
-            const int u = (int)(t - ncol), rg = u / wide;
-            j = u - rg * wide - GC;
+            const long long u = t - ncol;
+            const int rg = (int)(u / wide);
+            j = (int)(u - (long long)rg * wide) - GC;
             i = rg < GR ? rg - GR : nx + rg - GR;
         }
         const int si = ((i % nx) + nx) % nx, sj = ((j % ny) + ny) % ny;

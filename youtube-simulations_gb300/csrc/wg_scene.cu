@@ -333,17 +333,20 @@ wg_status wg_scene_create(const wg_params *p, int32_t precision, int32_t coef_mo
         if (e != cudaSuccess) { delete s; return cuda_fail(e, "cudaStreamCreate"); }
         s->own_stream = true;
     }
-    bool ok = true;
-    for (int k = 0; k < 2 && ok; k++)
-        ok = scene_alloc_field(s, &s->f[k]) == WG_OK && (precision != WG_FP32 || scene_alloc_field(s, &s->g[k]) == WG_OK);
-    if (ok && coef_mode == WG_COEF_TABLE)
-        ok = scene_alloc_field(s, &s->tcc) == WG_OK &&
-             ((p->b_cond != WG_BC_ABSORBING && p->b_cond != WG_BC_VPER_HABS) || scene_alloc_field(s, &s->tc) == WG_OK);
-    if (!ok) {
+    st = WG_OK;
+    for (int k = 0; k < 2 && !st; k++) {
+        st = scene_alloc_field(s, &s->f[k]);
+        if (!st && precision == WG_FP32) st = scene_alloc_field(s, &s->g[k]);
+    }
+    if (!st && coef_mode == WG_COEF_TABLE) {
+        st = scene_alloc_field(s, &s->tcc);
+        if (!st && (p->b_cond == WG_BC_ABSORBING || p->b_cond == WG_BC_VPER_HABS)) st = scene_alloc_field(s, &s->tc);
+    }
+    if (st) {
         const std::string msg = wg_last_error();
         wg_scene_destroy(s);
         set_error("%s", msg.c_str());
-        return WG_ERR_CUDA;
+        return st;
     }
     cudaError_t e = cudaSuccess;
     for (uint32_t **m : {&s->act, &s->nz}) {
