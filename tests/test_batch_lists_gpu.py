@@ -41,3 +41,32 @@ def test_lists_of_every_length(bc, count, nx, ny, mode):
             got = b.download(slots[k])
             for x, y in zip(got, ref):
                 assert np.array_equal(np.asarray(x).view(np.int64), np.asarray(y).view(np.int64)), k
+
+
+@pytest.mark.parametrize("bc", [P.BC_PERIODIC, P.BC_DIRICHLET, P.BC_ABSORBING])
+@pytest.mark.parametrize("count,nx,ny", [(420, 61, 129), (420, 61, 241), (6, 131, 257), (3, 40, 113)])
+@pytest.mark.parametrize("mode", [6, 5, -1])
+def test_deep_passes_near_the_stability_limit(bc, count, nx, ny, mode):
+    """Frames cut into passes of the greatest depth (6, 12 and 16 updates), each reading what the one before
+    wrote, at Courant numbers where a wrong value at the far end of a halo is not lost in
+    rounding; one column in the last group of four, lists with and without tickets."""
+    with W.Batch(P.FP32) as b:
+        b.set_skew(mode)
+        inst = []
+        for k in range(count):
+            p, phi, psi, xy = instance(k, nx, ny, bc)
+            p.courant = (0.65, 0.5, 0.3)[k % 3]
+            inst.append((p, phi, psi, xy))
+        slots = [b.add(*i) for i in inst]
+        for n in (6, 12, 16):
+            b.step(n)
+        for k in range(0, count, max(1, count // 9)):
+            p, phi, psi, xy = inst[k]
+            with W.Scene(p, P.FP32, P.COEF_MASK) as s:
+                s.set_blocking(1)
+                s.upload(phi, psi, xy)
+                s.step(34)
+                ref = s.download()
+            assert np.isfinite(ref[0]).all()
+            for x, y in zip(b.download(slots[k]), ref):
+                assert np.array_equal(np.asarray(x).view(np.int64), np.asarray(y).view(np.int64)), k

@@ -54,3 +54,34 @@ def test_passes_match_single_updates(nx, ny, coef, kw):
                 assert s.blocking() == blocking
         for a, b in zip(got, ref):
             assert np.array_equal(a, b), blocking
+
+
+@pytest.mark.parametrize("ny", [109, 113, 114, 115, 117, 225, 241, 257, 717])
+@pytest.mark.parametrize("courant", [0.3, 0.5, 0.65])
+@pytest.mark.parametrize("coef,kw", [(P.COEF_MASK, dict()), (P.COEF_TABLE, dict(twospeeds=1, courantb=0.2, gammab=1e-4)),
+                                     (P.COEF_MASK, dict(floor_clamp=1, vmax=2.0))])
+def test_ghosts_of_the_last_group_of_columns(ny, courant, coef, kw):
+    """Passes that read the ghosts another pass wrote, at Courant numbers near the stability limit, where
+    a wrong value at the far end of a halo is not lost in rounding: widths that leave the last
+    group of four columns one, two, three and four cells, in one tile and in several."""
+    nx = 45
+    rng = np.random.default_rng(ny)
+    n = nx * ny
+    p = P.make_params(nx, ny, b_cond=P.BC_PERIODIC, courant=courant, **kw)
+    xy = (rng.random(n) < 0.9).astype(np.int16)
+    f = (rng.standard_normal(n), rng.standard_normal(n), xy) + (scenes.tables(p, xy) if coef == P.COEF_TABLE else ())
+
+    def run(blocking):
+        out = []
+        with W.Scene(p, P.FP32, coef) as s:
+            s.upload(*f)
+            s.set_blocking(*blocking)
+            for steps in (6, 12, 18, 11):
+                s.step(steps)
+                out += s.download(native=True)
+        return out
+    ref = run((1,))
+    assert all(np.isfinite(a).all() for a in ref)
+    for blocking in [(5, 8, 1), (6, 8, 1), (6, 64, 1)]:
+        for a, b in zip(run(blocking), ref):
+            assert np.array_equal(a, b), blocking

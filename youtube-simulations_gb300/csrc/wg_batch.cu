@@ -236,14 +236,14 @@ __global__ void __launch_bounds__(128, 4) k_batch_step64(const BatchHdr *__restr
 // ordering.
 __device__ __forceinline__ void ghost_fill(float *f0, float *f1, int nx, int ny, int pitch, long long t0, long long nt)
 {
-    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
-    const int wide = ny + 2 * GC, ncol = 2 * GC * nx;
+    constexpr int GC = BATCH_GHOST_COLS, GT = GC + BATCH_GHOST_COLS_R, GR = BATCH_GHOST_ROWS;
+    const int wide = ny + GT, ncol = GT * nx;
     const long long total = ncol + 2LL * GR * wide;
     for (long long t = t0; t < total; t += nt) {
         int i, j;
         if (t < ncol) {  // the ghost columns of the real rows
-            i = (int)t / (2 * GC);
-            const int g = (int)t - i * 2 * GC;
+            i = (int)t / GT;
+            const int g = (int)t - i * GT;
             j = g < GC ? g - GC : ny + g - GC;
         } else {  // the ghost rows, over the extended width
             const long long u = t - ncol;
@@ -280,7 +280,7 @@ __global__ void k_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch)
 }
 void launch_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch, cudaStream_t st)
 {
-    const long long total = 2LL * BATCH_GHOST_COLS * nx + 2LL * BATCH_GHOST_ROWS * (ny + 2 * BATCH_GHOST_COLS);
+    const long long gt = BATCH_GHOST_COLS + BATCH_GHOST_COLS_R, total = gt * nx + 2LL * BATCH_GHOST_ROWS * (ny + gt);
     k_grid_ghosts<<<(unsigned)std::min(608LL, (total + 127) / 128), 128, 0, st>>>(f0, f1, nx, ny, pitch);
 }
 

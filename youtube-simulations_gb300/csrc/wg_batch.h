@@ -38,13 +38,20 @@ struct BatchHdr {
 
 constexpr int BATCH_CLASSES = 16;   // size classes: floor(log2(cells)) - 10, clamped to 0..15
 
-// Ghost layout of a periodic scene taking skewed passes: every field row carries
-// BATCH_GHOST_COLS copies of the opposite side's columns on each side, and the field
-// BATCH_GHOST_ROWS copies of the opposite rows above row 0 and below row nx-1, so that a
+// Ghost layout of a periodic scene taking skewed passes: every field row carries copies of the
+// opposite side's columns, BATCH_GHOST_COLS on the left and BATCH_GHOST_COLS_R on the right, and the
+// field BATCH_GHOST_ROWS copies of the opposite rows above row 0 and below row nx-1, so that a
 // pass reads its wrapped halo as ordinary neighbours.  The scene's pointers address cell
 // (0, 0); the ghosts sit at negative offsets and in the row padding.  Mask planes carry one
 // ghost word on the left of every row and the same ghost rows.
+//
+// A pass stores whole groups of four columns, so the last group of a row also holds the ghost
+// columns ny .. batch_group_end(ny) - 1.  They are right because their halo is there: the last of
+// them, at most ny+2, depends on columns up to ny+8 at depth 6, hence one ghost column more on the right.
 constexpr int BATCH_GHOST_COLS = 8;   // the widest column halo of a pass (depth 5..6)
+constexpr int BATCH_GHOST_COLS_R = BATCH_GHOST_COLS + 1;
+static_assert(WG_SKEW_MAX_K + 3 <= BATCH_GHOST_COLS_R, "the last group's ghost columns need their halo");
+__host__ __device__ inline int batch_group_end(int ny) { return (ny + 3) & ~3; }
 constexpr int BATCH_GHOST_ROWS = 7;   // the deepest row halo of a pass (depth 6 + 1)
 constexpr int BATCH_GROUPS = WG_SKEW_MAX_K + 1;
 

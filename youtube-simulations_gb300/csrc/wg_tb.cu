@@ -862,14 +862,16 @@ __global__ void __launch_bounds__(32 * P, skew_min_blocks(P))
 // The ghost cells that mirror the rows [i_s, i_e) and columns [lo, hi) of a wrapped scene's new
 // fields, by the team that stored them: a cell within BATCH_GHOST_COLS of the left or right edge or
 // BATCH_GHOST_ROWS of the top or bottom one goes to every place of the extended grid that wraps to
-// it.  (The last group of four columns may reach past ny-1; the cells it stores there are the
-// same values.)  A kernel before each pass did this over the whole batch, 22 us with 48 scenes, and
+// it, but for the ghost columns of a real row's last group of four, which the team of the last tile
+// stores with that group: every cell has one writer.
+// A kernel before each pass did this over the whole batch, 22 us with 48 scenes, and
 // kept passes from overlapping: 48 scenes of 256 to 960 a side, half of them periodic, 10 updates:
 // 224 to 195 us.
 __device__ __noinline__ void skew_images(float *f0, float *f1, int nx, int ny, int pitch, int i_s, int i_e, int lo, int hi,
                                          int t0, int nt)
 {
-    constexpr int GC = BATCH_GHOST_COLS, GR = BATCH_GHOST_ROWS;
+    constexpr int GC = BATCH_GHOST_COLS, GX = BATCH_GHOST_COLS_R, GR = BATCH_GHOST_ROWS;
+    const int ge = batch_group_end(ny);
     // cells t0, t0 + nt, .. of an nr x nc block whose cell (r, c) is (row(r), col(c)): the loads of
     // four cells before their stores while there are four, then one by one
     const auto cells = [&](auto u, int t, int nc, auto row, auto col) {
@@ -888,8 +890,8 @@ __device__ __noinline__ void skew_images(float *f0, float *f1, int nx, int ny, i
 #pragma unroll
         for (int k = 0; k < U; k++)
             for (int i = rr[k] - nx * ((rr[k] + GR) / nx); i < nx + GR; i += nx)
-                for (int j = cc[k] - ny * ((cc[k] + GC) / ny); j < ny + GC; j += ny)
-                    if (i != rr[k] || j != cc[k]) {
+                for (int j = cc[k] - ny * ((cc[k] + GC) / ny); j < ny + GX; j += ny)
+                    if (i != rr[k] || (j != cc[k] && (j < ny || j >= ge))) {
                         f0[(long long)i * pitch + j] = x[k];
                         f1[(long long)i * pitch + j] = v[k];
                     }
@@ -900,7 +902,7 @@ __device__ __noinline__ void skew_images(float *f0, float *f1, int nx, int ny, i
         for (; t < nr * nc; t += nt) cells(std::integral_constant<int, 1>(), t, nc, row, col);
     };
     // the two bands of columns, all rows
-    const int wa = max(0, min(hi, GC) - lo), b0 = max(max(lo, ny - GC), lo + wa), wb = max(0, hi - b0), wc = wa + wb;
+    const int wa = max(0, min(hi, GX) - lo), b0 = max(max(lo, ny - GC), lo + wa), wb = max(0, hi - b0), wc = wa + wb;
     if (wc > 0) block(i_e - i_s, wc, [&](int r) { return i_s + r; }, [&](int q) { return q < wa ? lo + q : b0 + q - wa; });
     // the two bands of rows, the columns between
     const int na = max(0, min(i_e, GR) - i_s), r0 = max(max(i_s, nx - GR), i_s + na), nb = max(0, i_e - r0);
