@@ -50,3 +50,33 @@ def test_page_locked_rows(nx, ny, prec, native, offsets):
         both, _ = pinned(n, 1, dt)  # the same rows twice: psi's copy comes last
         W.check(calls[0](both.ctypes.data, both.ctypes.data))
         assert np.array_equal(both, ref[1])
+
+
+@pytest.mark.parametrize("prec,native,shift", [(P.FP32, True, 1), (P.FP32, True, 2), (P.FP32, False, 1), (P.FP32, False, 4),
+                                               (P.FP64, False, 2), (P.FP64, False, 4)])
+def test_page_locked_rows_not_aligned_to_their_cells(prec, native, shift):
+    """Rows at any byte address are copied, not accessed as cells in place: the same values, down and up."""
+    nx, ny = 13, 37
+    n = nx * ny
+    dt = np.dtype(np.float32 if native else np.float64)
+    code = P.FP32 if native else P.FP64
+    rng = np.random.default_rng(shift)
+    f = rng.standard_normal(n), rng.standard_normal(n)
+    whole = [torch.zeros(n * dt.itemsize + 16, dtype=torch.uint8, pin_memory=True).numpy() for _ in range(2)]
+    rows = [w[shift:shift + n * dt.itemsize] for w in whole]
+    with W.Scene(P.make_params(nx, ny, courant=0.1), prec, P.COEF_MASK) as s, W.Batch(prec) as b:
+        s.upload(*f, np.ones(n, np.int16))
+        s.step(3)
+        want = s.download(native=native)
+        W.check(W.lib().wg_scene_download(s.h, rows[0].ctypes.data, rows[1].ctypes.data, code))
+        got = [r.copy().view(dt) for r in rows]
+        assert all(np.array_equal(g, w) for g, w in zip(got, want))
+        W.check(W.lib().wg_scene_upload_state(s.h, rows[0].ctypes.data, rows[1].ctypes.data, code))
+        up = s.download(native=native)
+        s.upload_state(*want)
+        assert all(np.array_equal(g, w) for g, w in zip(up, s.download(native=native)))
+        if not native:
+            slot = b.add(s.params, *f, np.ones(n, np.int16))
+            b.step(3)
+            W.check(W.lib().wg_batch_download(b.h, slot, rows[0].ctypes.data, rows[1].ctypes.data))
+            assert all(np.array_equal(r.copy().view(dt), w) for r, w in zip(rows, b.download(slot)))

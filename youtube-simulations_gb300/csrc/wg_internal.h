@@ -96,10 +96,16 @@ template <class H> void launch_state_in32(int nx, int ny, int pitch, const H *ph
 // Fields (x0, y0), or (x1, y1) where *sel is not 0, to dense (phi, psi) rows; either may be NULL
 template <class T, class H> void launch_state_out(int nx, int ny, int pitch, const T *x0, const T *y0, const T *x1,
                                                   const T *y1, const int *sel, H *phi, H *psi, cudaStream_t st);
+// The device address of n page-locked cells that kernels may access as H, or nullptr (rows that are
+// not aligned to their cells too: a copy takes any address, a kernel does not).
+template <class H> inline H *mapped_cells(H *p, size_t n)
+{
+    return (uintptr_t)p % alignof(H) ? nullptr : (H *)mapped_host(p, n * sizeof(H));
+}
 // The rows as device addresses of page-locked memory (written in place); false when they are not
 template <class H> inline bool mapped_rows(H *&phi, H *&psi, size_t n)
 {
-    H *a = phi ? (H *)mapped_host(phi, n * sizeof(H)) : nullptr, *b = psi ? (H *)mapped_host(psi, n * sizeof(H)) : nullptr;
+    H *a = phi ? mapped_cells(phi, n) : nullptr, *b = psi ? mapped_cells(psi, n) : nullptr;
     if ((phi && !a) || (psi && !b)) return false;
     if (a && b && a < b + n && b < a + n) return false;  // they overlap: psi's copy comes last
     phi = a;

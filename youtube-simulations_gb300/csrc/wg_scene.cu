@@ -120,7 +120,7 @@ template <class H>
 static wg_status upload_state32(wg_scene *s, const H *phi, const H *psi, bool sync)
 {
     const size_t n = (size_t)s->prm.nx * s->prm.ny, bytes = n * sizeof(H);
-    const H *mphi = (const H *)mapped_host(phi, bytes), *mpsi = (const H *)mapped_host(psi, bytes);
+    const H *mphi = mapped_cells(phi, n), *mpsi = mapped_cells(psi, n);
     if (mphi && mpsi) {
         launch_state_in32<H>(s->prm.nx, s->prm.ny, s->pitch, mphi, mpsi, (float *)s->f[s->cur],
                              (float *)s->f[1 - s->cur], s->st);
