@@ -4,6 +4,7 @@ everything between the steps that writes the fields, the mask or the tables: a p
 fields, a new domain, single updates."""
 import numpy as np
 import pytest
+import torch
 
 from youtube_simulations_gb300 import params as P
 from youtube_simulations_gb300 import scenes
@@ -85,3 +86,47 @@ def test_ghosts_of_the_last_group_of_columns(ny, courant, coef, kw):
     for blocking in [(5, 8, 1), (6, 8, 1), (6, 64, 1)]:
         for a, b in zip(run(blocking), ref):
             assert np.array_equal(a, b), blocking
+
+
+def recorded(stream, call):
+    """`call` recorded as a graph on the (torch) stream; it does not run."""
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        g.capture_begin()
+        try:
+            call()
+        finally:
+            g.capture_end()
+    return g
+
+
+def replay(stream, g):
+    with torch.cuda.stream(stream):
+        g.replay()
+
+
+@pytest.mark.parametrize("blocking", [None, (6, 8, 1), (5, 64, 1)])
+@pytest.mark.parametrize("steps", [6, 10])
+def test_recorded_before_the_first_call(blocking, steps):
+    """A call may be recorded on a periodic scene that has not been stepped, and so not tuned, yet."""
+    nx, ny = 37, 131
+    n = nx * ny
+    rng = np.random.default_rng(5)
+    p = P.make_params(nx, ny, b_cond=P.BC_PERIODIC, courant=0.5, twospeeds=1, courantb=0.3)
+    f = rng.standard_normal(n), rng.standard_normal(n), (rng.random(n) < 0.9).astype(np.int16)
+    with W.Scene(p, P.FP32, P.COEF_MASK) as s:
+        s.set_blocking(1)
+        s.upload(*f)
+        s.step(2 * steps)
+        want = s.download()
+    st = torch.cuda.Stream()
+    with W.Scene(p, P.FP32, P.COEF_MASK, stream=st.cuda_stream) as s:
+        s.upload(*f)
+        if blocking:
+            s.set_blocking(*blocking)
+        g = recorded(st, lambda: s.step(steps))
+        for _ in range(2):
+            replay(st, g)
+        got = s.download()
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)

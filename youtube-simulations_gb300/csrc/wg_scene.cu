@@ -228,6 +228,15 @@ static wg_status single_update(wg_scene *s)
     return WG_OK;
 }
 
+// Whether the scene's stream is recording a graph.
+wg_status scene_recording(const wg_scene *s, bool *rec)
+{
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    WG_CUDA(cudaStreamIsCapturing(s->st, &cap));
+    *rec = cap != cudaStreamCaptureStatusNone;
+    return WG_OK;
+}
+
 template <class T>
 wg_status scene_step_impl(wg_scene *s, int nsteps)
 {
@@ -236,13 +245,14 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
         return WG_ERR_STATE;
     }
     const int k = s->tb_k;
-    // probes sample every update; the TMA tiles do not wrap
-    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1);
     // a recorded call may be replayed after other calls have changed the fields or the mask: it
     // fills the ghosts itself, and leaves them to the next call
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (tb && s->wrap) WG_CUDA(cudaStreamIsCapturing(s->st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) s->ghosts_ok = s->mask_ghosts_ok = false;
+    bool rec = false;
+    if (s->wrap)
+        if (wg_status st = scene_recording(s, &rec)) return st;
+    if (rec) s->ghosts_ok = s->mask_ghosts_ok = false;
+    // probes sample every update; the TMA tiles do not wrap; a task list cannot be made while recording
+    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1) && !(rec && !tb_ready(s, nsteps));
     if (tb) {
         wg_status st = tb_prepare(s, nsteps);
         if (st) return st;
@@ -260,7 +270,7 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
             nsteps--;
         }
     }
-    if (cap != cudaStreamCaptureStatusNone) s->ghosts_ok = s->mask_ghosts_ok = false;
+    if (rec) s->ghosts_ok = s->mask_ghosts_ok = false;
     WG_CUDA(cudaGetLastError());
     return WG_OK;
 }
@@ -550,7 +560,13 @@ wg_status wg_scene_step(wg_scene *s, int32_t nsteps)
     if (!s) { set_error("NULL scene"); return WG_ERR_INVALID; }
     if (!s->uploaded) { set_error("upload the scene before stepping"); return WG_ERR_STATE; }
     if (nsteps < 0) { set_error("negative step count"); return WG_ERR_INVALID; }
-    if (s->tb_k == 0) autotune_scene(s);
+    if (s->tb_k == 0) {
+        // a periodic scene's call may be recorded before anything has been tuned: single updates then
+        bool rec = false;
+        if (s->wrap)
+            if (wg_status st = scene_recording(s, &rec)) return st;
+        if (!rec) autotune_scene(s);
+    }
     return s->prec == WG_FP32 ? scene_step_impl<float>(s, nsteps) : scene_step_impl<double>(s, nsteps);
 }
 

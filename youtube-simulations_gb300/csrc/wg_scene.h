@@ -69,11 +69,13 @@ wg_status scene_alloc_dense_stage(wg_scene *s, size_t bytes);
 void *scene_field_base(const wg_scene *s, void *f);  // the allocation of a field, or nullptr
 wg_status scene_alloc_field(wg_scene *s, void **f);  // zeroed, in the scene's layout
 size_t scene_device_bytes(const wg_params &p, int prec, int coef);
+wg_status scene_recording(const wg_scene *s, bool *rec);
 template <class T> wg_status scene_step_impl(wg_scene *s, int nsteps);
 // temporal blocking (wg_tb.cu)
 bool tb_supported(const wg_scene *s);
 template <class T> wg_status tb_pass(wg_scene *s, int k);
 int tb_pass_depth(int k, int remaining);
+bool tb_ready(const wg_scene *s, int n);  // the task lists of a call of n updates are there (skewed passes)
 wg_status tb_prepare(wg_scene *s, int n);
 wg_status scene_check_flag(wg_scene *s);
 void autotune_scene(wg_scene *s);

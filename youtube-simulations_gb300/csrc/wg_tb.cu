@@ -1511,6 +1511,16 @@ int tb_pass_depth(int k, int remaining)
     return (remaining + n - 1) / n;
 }
 
+bool tb_ready(const wg_scene *s, int n)
+{
+    while (n > 0) {
+        const int d = tb_pass_depth(s->tb_k, n);
+        if (d >= 2 && !(d <= WG_SKEW_MAX_K && s->skew[d].dev && s->skew[d].min_rows == s->tile_i)) return false;
+        n -= std::max(d, 1);
+    }
+    return true;
+}
+
 // ---------------------------------------------------------------------------
 // Autotuner: temporal-block depth and tile width per size class, measured once per
 // (size class, coefficient mode) with CUDA events on a copy of the scene's state.
