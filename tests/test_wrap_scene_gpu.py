@@ -130,3 +130,37 @@ def test_recorded_before_the_first_call(blocking, steps):
         got = s.download()
     for a, b in zip(got, want):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kind", ["step", "pulse", "state"])
+def test_replays_between_calls(kind):
+    """A replayed graph changes the fields without notice: the next call's ghosts are the new fields'."""
+    nx, ny = 37, 131
+    n = nx * ny
+    rng = np.random.default_rng(6)
+    p = P.make_params(nx, ny, b_cond=P.BC_PERIODIC, courant=0.5, twospeeds=1, courantb=0.3)
+    f = rng.standard_normal(n), rng.standard_normal(n), (rng.random(n) < 0.9).astype(np.int16)
+    rows = [torch.from_numpy(rng.standard_normal(n).astype(np.float32)).pin_memory() for _ in range(2)]
+    st = torch.cuda.Stream()
+
+    def call(s):
+        if kind == "step":
+            s.step(3)  # depth 2: a pass and a single update, so the fields return to their buffers
+        elif kind == "pulse":  # over a corner
+            s.add_circular_wave(1.0, -1.98, 1.1, variance=0.05)
+        else:
+            W.check(W.lib().wg_scene_upload_state(s.h, rows[0].data_ptr(), rows[1].data_ptr(), P.FP32))
+
+    def run(blocking, as_graph):
+        with W.Scene(p, P.FP32, P.COEF_MASK, stream=st.cuda_stream) as s:
+            s.upload(*f)
+            s.set_blocking(*blocking)
+            s.step(4)
+            g = recorded(st, lambda: call(s)) if as_graph else None
+            for _ in range(3):
+                replay(st, g) if as_graph else call(s)
+                s.step(4)
+            return s.download(native=True)
+    want = run((1,), False)
+    for a, b in zip(run((2, 8, 1), True), want):
+        assert np.array_equal(a, b)

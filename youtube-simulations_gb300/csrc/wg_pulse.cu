@@ -108,6 +108,8 @@ extern "C" wg_status wg_scene_add_circular_wave(wg_scene *s, double init_amp, do
     wg_status st = pulse_args(s->prm, s->pitch, s->dp.wpitch, init_amp, factor, x, y, variance, wavelength, &a);
     if (st) return st;
     void *phi = s->f[s->cur];
+    bool rec = false;
+    if ((st = scene_recording(s, &rec))) return st;
     s->ghosts_ok = false;
     if (s->prec == WG_FP32)
         launch_add_circular_wave<float>(a, (float *)phi, (float *)s->f[1 - s->cur], nullptr, s->nz, s->st);

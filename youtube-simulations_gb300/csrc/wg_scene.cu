@@ -228,12 +228,14 @@ static wg_status single_update(wg_scene *s)
     return WG_OK;
 }
 
-// Whether the scene's stream is recording a graph.
-wg_status scene_recording(const wg_scene *s, bool *rec)
+// Whether the stream of a periodic scene is recording a graph (others need not know).
+wg_status scene_recording(wg_scene *s, bool *rec)
 {
+    *rec = false;
+    if (!s->wrap) return WG_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     WG_CUDA(cudaStreamIsCapturing(s->st, &cap));
-    *rec = cap != cudaStreamCaptureStatusNone;
+    if (cap != cudaStreamCaptureStatusNone) *rec = s->recorded = true;
     return WG_OK;
 }
 
@@ -246,11 +248,12 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
     }
     const int k = s->tb_k;
     // a recorded call may be replayed after other calls have changed the fields or the mask: it
-    // fills the ghosts itself, and leaves them to the next call
+    // fills the ghosts itself.  Its replays change the fields without notice, so that from then on
+    // every call does
     bool rec = false;
-    if (s->wrap)
-        if (wg_status st = scene_recording(s, &rec)) return st;
-    if (rec) s->ghosts_ok = s->mask_ghosts_ok = false;
+    if (wg_status st = scene_recording(s, &rec)) return st;
+    if (s->recorded) s->ghosts_ok = false;
+    if (rec) s->mask_ghosts_ok = false;
     // probes sample every update; the TMA tiles do not wrap; a task list cannot be made while recording
     const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1) && !(rec && !tb_ready(s, nsteps));
     if (tb) {
@@ -270,7 +273,7 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
             nsteps--;
         }
     }
-    if (rec) s->ghosts_ok = s->mask_ghosts_ok = false;
+    if (rec) s->mask_ghosts_ok = false;
     WG_CUDA(cudaGetLastError());
     return WG_OK;
 }
@@ -472,6 +475,8 @@ wg_status wg_scene_upload_state(wg_scene *s, const void *phi, const void *psi, i
     const void *src[2] = {phi, psi};
     if (!s->has_mask) { set_error("upload or build the mask first"); return WG_ERR_STATE; }
     if (host_precision != WG_FP32 && host_precision != WG_FP64) { set_error("unknown host precision"); return WG_ERR_INVALID; }
+    bool rec = false;
+    if (wg_status st = scene_recording(s, &rec)) return st;
     s->uploaded = true;
     s->ghosts_ok = false;
     if (s->prec == WG_FP32) {  // stream-ordered for FP32 host rows, as for same-precision copies below
@@ -563,8 +568,7 @@ wg_status wg_scene_step(wg_scene *s, int32_t nsteps)
     if (s->tb_k == 0) {
         // a periodic scene's call may be recorded before anything has been tuned: single updates then
         bool rec = false;
-        if (s->wrap)
-            if (wg_status st = scene_recording(s, &rec)) return st;
+        if (wg_status st = scene_recording(s, &rec)) return st;
         if (!rec) autotune_scene(s);
     }
     return s->prec == WG_FP32 ? scene_step_impl<float>(s, nsteps) : scene_step_impl<double>(s, nsteps);

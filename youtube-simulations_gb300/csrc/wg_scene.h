@@ -26,7 +26,9 @@ struct wg_scene {
     // to its fields, tables and masks address cell (0, 0), field_off cells and mask_off words into
     // allocations of field_bytes and mask_bytes.  ghosts_ok: the current fields hold their
     // ghosts; mask_ghosts_ok: the active plane and tcc do.
-    bool wrap = false, ghosts_ok = false, mask_ghosts_ok = false;
+    // recorded: a call that changes the fields has been recorded into a graph, whose
+    // replays may change them at any time.
+    bool wrap = false, ghosts_ok = false, mask_ghosts_ok = false, recorded = false;
     size_t field_off = 0, mask_off = 0, field_bytes = 0, mask_bytes = 0;
     uint32_t *act = nullptr, *nz = nullptr;
     int has_ghosts = 0;
@@ -69,7 +71,7 @@ wg_status scene_alloc_dense_stage(wg_scene *s, size_t bytes);
 void *scene_field_base(const wg_scene *s, void *f);  // the allocation of a field, or nullptr
 wg_status scene_alloc_field(wg_scene *s, void **f);  // zeroed, in the scene's layout
 size_t scene_device_bytes(const wg_params &p, int prec, int coef);
-wg_status scene_recording(const wg_scene *s, bool *rec);
+wg_status scene_recording(wg_scene *s, bool *rec);
 template <class T> wg_status scene_step_impl(wg_scene *s, int nsteps);
 // temporal blocking (wg_tb.cu)
 bool tb_supported(const wg_scene *s);
