@@ -145,7 +145,7 @@ def test_replays_between_calls(kind):
 
     def call(s):
         if kind == "step":
-            s.step(3)  # depth 2: a pass and a single update, so the fields return to their buffers
+            s.step(4)
         elif kind == "pulse":  # over a corner
             s.add_circular_wave(1.0, -1.98, 1.1, variance=0.05)
         else:
@@ -163,4 +163,42 @@ def test_replays_between_calls(kind):
             return s.download(native=True)
     want = run((1,), False)
     for a, b in zip(run((2, 8, 1), True), want):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("nx,ny,blocking", [(37, 131, (6, 8, 1)), (37, 131, (3, 16, 1)), (700, 45, None)])
+@pytest.mark.parametrize("steps", [2, 4, 6, 10, 18])
+@pytest.mark.parametrize("warm", [True, False])
+def test_replays_advance_the_scene(nx, ny, blocking, steps, warm):
+    """A graph of an even number of updates leaves the fields in the buffers that it holds, as single updates
+    do, whether the scene was tuned and stepped before, and with other calls in between: steps of any
+    even length, another blocking (the graph keeps its task lists), a first tuning."""
+    n = nx * ny
+    rng = np.random.default_rng(7)
+    p = P.make_params(nx, ny, b_cond=P.BC_PERIODIC, courant=0.5, twospeeds=1, courantb=0.3)
+    f = rng.standard_normal(n), rng.standard_normal(n), (rng.random(n) < 0.9).astype(np.int16)
+    st = torch.cuda.Stream()
+
+    def run(blk, as_graph):
+        with W.Scene(p, P.FP32, P.COEF_MASK, stream=st.cuda_stream) as s:
+            s.upload(*f)
+            if blk:
+                s.set_blocking(*blk)
+            if warm:
+                s.step(steps)
+            g = recorded(st, lambda: s.step(steps)) if as_graph else None
+
+            def again():
+                replay(st, g) if as_graph else s.step(steps)
+            again()
+            again()
+            s.step(6)
+            again()
+            if as_graph:
+                s.set_blocking(6, 64, 1)
+            s.step(12)
+            again()
+            return s.download(native=True)
+    want = run((1,), False)
+    for a, b in zip(run(blocking, True), want):
         assert np.array_equal(a, b)

@@ -254,14 +254,19 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
     if (wg_status st = scene_recording(s, &rec)) return st;
     if (s->recorded) s->ghosts_ok = false;
     if (rec) s->mask_ghosts_ok = false;
-    // probes sample every update; the TMA tiles do not wrap; a task list cannot be made while recording
-    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1) && !(rec && !tb_ready(s, nsteps));
+    // probes sample every update; the TMA tiles do not wrap
+    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1);
     if (tb) {
         wg_status st = tb_prepare(s, nsteps);
         if (st) return st;
     }
+    // A pass swaps the fields' buffers once.  A graph holds the buffers of its recording, so on a
+    // periodic scene that has been recorded a call swaps them as often, to within an even number, as it
+    // has updates: whichever form a call takes, the fields are then where the graph expects them.
+    int passes = tb ? tb_passes(k, nsteps, s->recorded) : 0;
     while (nsteps > 0) {
-        const int d = tb ? tb_pass_depth(k, nsteps) : 0;
+        const int d = passes > 0 ? (nsteps + passes - 1) / passes : 0;
+        passes--;
         if (d >= 2) {
             wg_status st = tb_pass<T>(s, d);
             if (st) return st;
@@ -396,6 +401,7 @@ wg_status wg_scene_destroy(wg_scene *s)
                    s->nrec_dev};
     for (void *d : dev) if (d) cudaFree(d);
     for (auto &c : s->skew) if (c.dev) cudaFree(c.dev);
+    for (void *d : s->retired) cudaFree(d);
     if (s->hout) cudaFreeHost(s->hout);
     if (s->hstage) cudaFreeHost(s->hstage);
     if (s->own_stream && s->st) cudaStreamDestroy(s->st);

@@ -58,6 +58,7 @@ struct wg_scene {
     size_t rgb_bytes = 0;
     int tb_k = 0, tile_i = 0, tile_j = 0;
     SkewPlanCache skew[WG_SKEW_MAX_K + 1];  // task lists of the skewed kernel, by depth
+    std::vector<void *> retired;            // former lists that a recorded call may hold
     float *bv_osc = nullptr;   // oscillating values of the current step() call, [n][ny]
     double *bv_src = nullptr;  // point-source increments of the current step() call, [n]
     size_t bv_cap = 0;
@@ -76,8 +77,7 @@ template <class T> wg_status scene_step_impl(wg_scene *s, int nsteps);
 // temporal blocking (wg_tb.cu)
 bool tb_supported(const wg_scene *s);
 template <class T> wg_status tb_pass(wg_scene *s, int k);
-int tb_pass_depth(int k, int remaining);
-bool tb_ready(const wg_scene *s, int n);  // the task lists of a call of n updates are there (skewed passes)
+int tb_passes(int k, int n, bool parity);
 wg_status tb_prepare(wg_scene *s, int n);
 wg_status scene_check_flag(wg_scene *s);
 void autotune_scene(wg_scene *s);

@@ -1098,6 +1098,32 @@ static std::vector<int4> wrap_plan(const DevParams &p, int K, int min_rows, int 
     return out;
 }
 
+// A task list in device memory.  On a scene that is recorded its stream may be recording now: the
+// allocation is then made in the capture mode that allows it, and the copy on a stream of its own.
+static wg_status device_list(const std::vector<int4> &v, bool recorded, int4 **dev)
+{
+    const size_t bytes = v.size() * sizeof(int4);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaStream_t st = nullptr;
+    if (recorded) WG_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    int4 *d = nullptr;
+    cudaError_t e = cudaMalloc(&d, bytes);
+    if (e == cudaSuccess && recorded) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) {
+        e = recorded ? cudaMemcpyAsync(d, v.data(), bytes, cudaMemcpyHostToDevice, st)
+                     : cudaMemcpy(d, v.data(), bytes, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && recorded) e = cudaStreamSynchronize(st);
+    }
+    if (st) cudaStreamDestroy(st);
+    if (recorded) cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+        if (d) cudaFree(d);
+        return cuda_fail(e, "skewed task list");
+    }
+    *dev = d;
+    return WG_OK;
+}
+
 // Task list of (depth K, minimum rows L) for this scene, built once and kept on the device.
 static wg_status skew_tasks(wg_scene *s, int K, int L, const int4 **tasks, int *ntasks)
 {
@@ -1106,10 +1132,10 @@ static wg_status skew_tasks(wg_scene *s, int K, int L, const int4 **tasks, int *
     if (!c.dev || c.min_rows != L) {
         const int cap = skew_call(s->dp, nullptr, s->coef, K, nullptr, 0, s->st, s->wrap);
         const std::vector<int4> v = s->wrap ? wrap_plan(s->dp, K, L, cap) : skew_plan(s->dp, K, L, cap);
-        if (c.dev) cudaFree(c.dev);
+        if (c.dev && s->recorded) s->retired.push_back(c.dev);
+        else if (c.dev) cudaFree(c.dev);
         c.dev = nullptr;
-        WG_CUDA(cudaMalloc(&c.dev, v.size() * sizeof(int4)));
-        WG_CUDA(cudaMemcpy(c.dev, v.data(), v.size() * sizeof(int4), cudaMemcpyHostToDevice));
+        if (wg_status st = device_list(v, s->recorded, &c.dev)) return st;
         c.n = (int)v.size();
         c.min_rows = L;
     }
@@ -1501,24 +1527,16 @@ wg_status tb_pass<double>(wg_scene *, int)
     return WG_ERR_STATE;
 }
 
-int tb_pass_depth(int k, int remaining)
+// Passes of a call of n updates at depth k, each of n/passes updates, rounded up while they last; 0:
+// single updates.  The fewest passes of depth <= k, so that depths are equal to within one (10 updates
+// at k = 4: 4, 3, 3, at k = 6: 5, 5; 6 and a single update would be three launches).  parity: an even
+// number of passes for an even n, an odd one for an odd n (the last may then be a single update).
+int tb_passes(int k, int n, bool parity)
 {
-    // the fewest passes of depth <= k, of equal depth to within one (10 updates at k = 4: 4, 3, 3,
-    // at k = 6: 5, 5; 6 and a single update would be three launches); 0 = a single update
     const int m = std::min(k, 8);
-    if (m < 2 || remaining < 2) return 0;
-    const int n = (remaining + m - 1) / m;
-    return (remaining + n - 1) / n;
-}
-
-bool tb_ready(const wg_scene *s, int n)
-{
-    while (n > 0) {
-        const int d = tb_pass_depth(s->tb_k, n);
-        if (d >= 2 && !(d <= WG_SKEW_MAX_K && s->skew[d].dev && s->skew[d].min_rows == s->tile_i)) return false;
-        n -= std::max(d, 1);
-    }
-    return true;
+    if (m < 2 || n < 2) return 0;
+    const int q = (n + m - 1) / m;
+    return parity && ((q ^ n) & 1) ? q + 1 : q;
 }
 
 // ---------------------------------------------------------------------------
@@ -1561,6 +1579,7 @@ void autotune_scene(wg_scene *s)
         cudaMemcpyAsync(save[1], scene_field_base(s, s->f[1]), fb, cudaMemcpyDeviceToDevice, s->st);
         const long long t_save = s->time;
         const int cur_save = s->cur;
+        void *const bufs[] = {s->f[0], s->f[1], s->g[0], s->g[1]};  // the fields return to their buffers
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
@@ -1601,6 +1620,10 @@ void autotune_scene(wg_scene *s)
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         s->cur = cur_save;
+        for (int k = 0; k < 2; k++) {
+            s->f[k] = bufs[k];
+            s->g[k] = bufs[2 + k];
+        }
         cudaMemcpyAsync(scene_field_base(s, s->f[0]), save[0], fb, cudaMemcpyDeviceToDevice, s->st);
         cudaMemcpyAsync(scene_field_base(s, s->f[1]), save[1], fb, cudaMemcpyDeviceToDevice, s->st);
         cudaStreamSynchronize(s->st);
