@@ -202,3 +202,26 @@ def test_replays_advance_the_scene(nx, ny, blocking, steps, warm):
     want = run((1,), False)
     for a, b in zip(run(blocking, True), want):
         assert np.array_equal(a, b)
+
+
+def test_upload_that_fails_half_way():
+    """An upload without the tables it needs is refused after the mask has changed: the next steps take that
+    mask's ghosts too, as single updates take the mask."""
+    nx, ny = 37, 131
+    n = nx * ny
+    rng = np.random.default_rng(8)
+    p = P.make_params(nx, ny, b_cond=P.BC_PERIODIC, courant=0.5)
+    xy, other = ((rng.random(n) < q).astype(np.int16) for q in (0.9, 0.5))
+    f = rng.standard_normal(n), rng.standard_normal(n)
+    out = []
+    for blocking in [(1,), (6, 8, 1)]:
+        with W.Scene(p, P.FP32, P.COEF_TABLE) as s:
+            s.upload(*f, xy, *scenes.tables(p, np.ones_like(xy)))
+            s.set_blocking(*blocking)
+            s.step(12)
+            with pytest.raises(W.WaveGpuError):
+                s.upload(*f, other)
+            s.step(12)
+            out.append(s.download(native=True))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

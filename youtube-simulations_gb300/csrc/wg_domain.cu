@@ -379,6 +379,7 @@ extern "C" wg_status wg_scene_build_domain(wg_scene *s, int32_t domain, double l
         WG_CUDA(cudaMemcpy(dcirc, circles, sizeof(double) * 3 * d.ncirc, cudaMemcpyHostToDevice));
     }
     d.circ = dcirc;
+    s->mask_ghosts_ok = false;  // from here on the mask and the tables change, also when the call fails
     k_build_mask<<<dim3((d.wpitch + 127) / 128, d.nx), 128, 0, s->st>>>(d, s->act, s->nz);
     s->launches++;
     cudaError_t e = cudaGetLastError();
@@ -415,7 +416,6 @@ extern "C" wg_status wg_scene_build_domain(wg_scene *s, int32_t domain, double l
     s->has_ghosts = nrec > 0;
     s->xy_host.clear();
     s->has_mask = true;
-    s->mask_ghosts_ok = false;
     s->tb_k = 0;  // autotuned again for the new geometry
     return WG_OK;
 }

@@ -424,6 +424,8 @@ wg_status wg_scene_upload(wg_scene *s, const double *phi, const double *psi, con
             return WG_ERR_INVALID;
         }
     }
+    // from here on the mask, the tables and the fields may change, also when the call fails half way
+    s->ghosts_ok = s->mask_ghosts_ok = false;
     s->has_ghosts = has_neg;
     s->xy_host.assign(xy, xy + n);
     wg_status st = scene_alloc_dense_stage(s, n * sizeof(double));
@@ -469,7 +471,6 @@ wg_status wg_scene_upload(wg_scene *s, const double *phi, const double *psi, con
     s->time = 0;
     s->uploaded = true;
     s->has_mask = true;
-    s->ghosts_ok = s->mask_ghosts_ok = false;
     return WG_OK;
 }
 
