@@ -55,3 +55,27 @@ def test_amplitude_frames_at_the_palette_boundaries(nx, ny, prec, opts):
     may_differ = (np.abs(hv - np.round(hv)) < 1e-12) & (np.abs(u) > 1e-6)
     diff = np.any(img != ref, axis=-1)
     assert not np.any(diff & ~may_differ), np.argwhere(diff & ~may_differ)[:5]
+
+
+@pytest.mark.parametrize("prec", [P.FP32, P.FP64])
+@pytest.mark.parametrize("coef", [P.COEF_MASK, P.COEF_TABLE])
+@pytest.mark.parametrize("plot", [0, 1])
+def test_obstacle_fade_without_a_speed(prec, coef, plot):
+    """COURANT = 0: the obstacle fade is (0/0)^0.1 inside, drawn black, as 0 outside with COURANTB = 0."""
+    nx, ny = 17, 35
+    n = nx * ny
+    rng = np.random.default_rng(2)
+    L = frame_lut(4)
+    for courantb in (0.0, 0.1):
+        p = P.make_params(nx, ny, b_cond=P.BC_DIRICHLET, courant=0.0, courantb=courantb, twospeeds=1)
+        xy = (rng.random(n) < 0.6).astype(np.int16)
+        phi = rng.standard_normal(n).astype(np.float32).astype(np.float64)
+        tab = scenes.tables(p, xy)
+        with W.Scene(p, prec, coef) as s:
+            s.upload(phi, phi, xy, *(tab if coef == P.COEF_TABLE else ()))
+            img = s.frame_rgb8(L, size=1, plot=plot, fade_in_obstacle=True)
+        with np.errstate(all="ignore"):
+            ref = oracle.frame_rgb8(p, phi, xy, L, size=1, plot=plot, psi=phi, fade_in_obstacle=True)
+        assert np.array_equal(img[(xy.reshape(nx, ny) != 0).T], ref[(xy.reshape(nx, ny) != 0).T])
+        assert not img[(xy.reshape(nx, ny) != 0).T].any()
+        assert np.array_equal(img, ref)

@@ -25,7 +25,7 @@ __host__ __device__ inline int frame_tiles_y(int h) { return (h + FT_ROWS - 1) /
 struct FrameFast {
     float vshift, vscale, k, range, log_shift, log_scale, flux, inv_t;  // k = slope/scale; range includes the attenuation
     float es2, half, halfb;  // E_SCALE^2 and the energy's gradient factors inside and outside
-    float fade, inv_c2, ratio_b;  // FADE value; 1/COURANT^2, (COURANTB/COURANT)^2
+    float fade, inv_c2, ratio, ratio_b;  // FADE value; 1/COURANT^2, c2/c2 (1, or NaN), (COURANTB/COURANT)^2
     int plain;  // colours are palette bytes as they are: no fade, no obstacle fade
 };
 
@@ -45,6 +45,7 @@ inline FrameFast frame_fast(const wg_frame_params &fp, const DevParams &p)
     f.halfb = (float)p.ehalf_c2b;
     f.fade = (float)fp.fade_value;
     f.inv_c2 = (float)(1.0 / p.c2);  // (the server's kernel, whose scenes differ, uses none of p's)
+    f.ratio = (float)(p.c2 / p.c2);
     f.ratio_b = (float)(p.c2b / p.c2);
     f.plain = !fp.fade && !fp.fade_in_obstacle;
     return f;
@@ -102,7 +103,7 @@ static __device__ __noinline__ void frame_colour64(const wg_frame_params &fp, co
                                                    double cc, double c2, uint8_t *o)
 {
     double f = dim;
-    if (fp.fade_in_obstacle && cc != c2) f *= pow(cc / c2, 0.1);  // (pow of 1 is 1)
+    if (fp.fade_in_obstacle) f *= pow(cc / c2, 0.1);  // (NaN, and so black, where COURANT = 0 makes it 0/0)
     if (fp.fade) f *= fp.fade_value;
     for (int q = 0; q < 3; q++) {
         const double v = (double)lut[hue * 3 + q] * f;
