@@ -79,3 +79,68 @@ def test_obstacle_fade_without_a_speed(prec, coef, plot):
         assert np.array_equal(img[(xy.reshape(nx, ny) != 0).T], ref[(xy.reshape(nx, ny) != 0).T])
         assert not img[(xy.reshape(nx, ny) != 0).T].any()
         assert np.array_equal(img, ref)
+
+
+SCALES = [  # plot, frame parameters, scene parameters, size of phi, size of psi/phi - 1
+    (0, dict(vscale=1e30, slope=1e17, scale=1.0), dict(), 2e-47, 1.0),
+    (0, dict(vscale=1e-40, slope=1e17, scale=1.0), dict(), 1e23, 1.0),
+    (0, dict(slope=1.0, scale=1e46), dict(), 1e38, 1.0),
+    (0, dict(slope=1e40, scale=1.0), dict(), 1e-40, 1.0),
+    (1, dict(slope=1e30, scale=1.0), dict(e_scale=1e-25), 1e10, 1.0),
+    (2, dict(slope=1e30, scale=1.0), dict(e_scale=1e-25), 1e10, 1.0),
+    (3, dict(slope=1e30, scale=1.0), dict(e_scale=1e-25), 1e10, 1.0),
+    (4, dict(slope=1e19, log_scale=1e-20, log_shift=0.0), dict(), 1.0, 0.5),
+    (6, dict(flux_scale=1e38, slope=1e8, scale=1.0), dict(), 1e-23, 1.0),
+    (8, dict(slope=1e30, scale=1.0), dict(e_scale=1e-25), 1e10, 1.0),
+]
+
+
+@pytest.mark.parametrize("plot,kw,prm,size,rate", SCALES)
+def test_scales_beyond_fp32(plot, kw, prm, size, rate):
+    """Parameters and fields whose products, but not whose factors, are of ordinary size in FP32: the index
+    is the FP64 one.  The index of the log, mean and average modes follows from a logarithm or a
+    sum rounded a few times, so a pixel may differ only within 1e-10 of a boundary."""
+    nx, ny = 33, 70
+    n = nx * ny
+    rng = np.random.default_rng(9)
+    p = P.make_params(nx, ny, b_cond=P.BC_DIRICHLET, courant=0.1, courantb=0.06, twospeeds=1, **prm)
+    xy = (rng.random(n) < 0.6).astype(np.int16)
+    phi = size * rng.standard_normal(n)
+    psi = phi * (1.0 - rate * rng.standard_normal(n))
+    L = frame_lut(4)
+    kw = dict(dict(size=1, vshift=0.0), **kw)
+    with W.Scene(p, P.FP64, P.COEF_MASK) as s:
+        s.upload(phi, psi, xy)
+        img = s.frame_rgb8(L, plot=plot, **kw)
+    ref = oracle.frame_rgb8(p, phi, xy, L, plot=plot, psi=psi, **kw)
+    near = np.zeros((ny, nx), bool)
+    for shift in (-1e-10, 1e-10):  # where the palette index changes within 1e-10 of the amplitude
+        moved = oracle.frame_rgb8(p, phi, xy, np.repeat(np.arange(256), 3).reshape(256, 3).astype(np.uint8), plot=plot, psi=psi,
+                                  **dict(kw, color_range=0.8 * (1 + shift)))
+        near |= np.any(moved != oracle.frame_rgb8(p, phi, xy, np.repeat(np.arange(256), 3).reshape(256, 3).astype(np.uint8),
+                                                  plot=plot, psi=psi, **kw), axis=-1)
+    assert len(np.unique(ref.reshape(-1, 3), axis=0)) > 1
+    diff = np.any(img != ref, axis=-1)
+    assert not np.any(diff & ~near), (int(diff.sum()), int(near.sum()))
+
+
+@pytest.mark.parametrize("coef", [P.COEF_MASK, P.COEF_TABLE])
+@pytest.mark.parametrize("courantb", [5.5e-23, 1e-21, 1e-19, 1e-15, 1e-12])
+def test_obstacle_fade_of_tiny_speeds(coef, courantb):
+    nx, ny = 33, 70
+    n = nx * ny
+    rng = np.random.default_rng(10)
+    p = P.make_params(nx, ny, b_cond=P.BC_DIRICHLET, courant=0.1, courantb=courantb, twospeeds=1)
+    xy = (rng.random(n) < 0.3).astype(np.int16)
+    phi = rng.standard_normal(n)
+    tcc, tc, tg = scenes.tables(p, xy)
+    tcc = tcc * (1.0 + rng.random(n)) if coef == P.COEF_TABLE else tcc
+    L = frame_lut(4)
+    kw = dict(size=1, fade=True, fade_value=0.4 / (courantb / 0.1) ** 0.2, fade_in_obstacle=True)
+    with W.Scene(p, P.FP64, coef) as s:
+        s.upload(phi, phi, xy, *((tcc, tc, tg) if coef == P.COEF_TABLE else ()))
+        img = s.frame_rgb8(L, **kw)
+    ref = oracle.frame_rgb8(p, phi, xy, L, tcc=tcc, **kw)
+    out = (xy.reshape(nx, ny) == 0).T  # (inside, the fade saturates every byte but 0)
+    assert len(np.unique(ref[out].reshape(-1, 3), axis=0)) > 10
+    assert np.array_equal(img, ref)

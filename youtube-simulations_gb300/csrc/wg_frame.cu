@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(FT_ROWS *FT_COLS) k_frame_rgb8(const __grid_co
                 if (fp.fade_in_obstacle) cc = (COEF == WG_COEF_TABLE) ? (double)tcc[c] : (m ? p.c2 : p.c2b);
                 // powf is within 4 ulp, its argument within 3e-7 (a tenth of which counts)
                 float ff32 = (float)dim * (fp.fade ? ff.fade : 1.f);
-                if (fp.fade_in_obstacle) ff32 *= powf((COEF == WG_COEF_TABLE) ? (float)tcc[c] * ff.inv_c2 : (m ? ff.ratio : ff.ratio_b), 0.1f);
+                if (fp.fade_in_obstacle) ff32 *= powf((COEF == WG_COEF_TABLE) ? fade_ratio((float)tcc[c], ff.inv_c2) : (m ? ff.ratio : ff.ratio_b), 0.1f);
                 if (!colour_fast(lut, hue, ff32, 8e-7f, o)) frame_colour64(fp, lut, hue, dim, cc, p.c2, o);
             }
         }

@@ -48,6 +48,14 @@ inline FrameFast frame_fast(const wg_frame_params &fp, const DevParams &p)
     f.ratio = (float)(p.c2 / p.c2);
     f.ratio_b = (float)(p.c2b / p.c2);
     f.plain = !fp.fade && !fp.fade_in_obstacle;
+    // The error bounds leave out what FP32 loses below its smallest numbers.  That does not matter while
+    // the factors of a value are 0 or within 1e-30..1e12; otherwise (k a NaN) every pixel takes FP64.
+    const auto fits = [](double v) { return v == 0.0 || (fabs(v) >= 1e-30 && fabs(v) <= 1e12); };
+    bool ok = fits(fp.slope / fp.scale) && fits(f.range);
+    if (fp.plot == WG_P_AMPLITUDE) ok = ok && fits(fp.vscale);
+    else ok = ok && fits(fp.log_scale) && fits(fp.flux_scale) && fits(f.inv_t) && fits(p.e_scale2) && fits(p.ehalf_c2) && fits(p.ehalf_c2b);
+    if (!ok) f.k = NAN;
+    if (!fits(p.c2b / p.c2)) f.ratio_b = NAN;
     return f;
 }
 
@@ -78,6 +86,14 @@ __device__ __forceinline__ float amplitude_fast(const FrameFast &f, float x, flo
     const float sx = f.vscale * x;
     *err = 4e-7f * (fabsf(f.vshift) + fabsf(sx));
     return f.vshift + sx;
+}
+
+// cc/c2 of the obstacle fade, NaN (the colour then takes FP64) where FP32 may have lost digits of cc,
+// c2 or the ratio to its smallest numbers.
+__device__ __forceinline__ float fade_ratio(float cc, float inv_c2)
+{
+    const float r = cc * inv_c2;
+    return inv_c2 >= 1e-30f && inv_c2 <= 1e30f && (cc == 0.f || (cc >= 1e-30f && r >= 1e-30f)) ? r : NAN;
 }
 
 // lut colour times f (known to within a relative rel), rounded, to o; false where the bound

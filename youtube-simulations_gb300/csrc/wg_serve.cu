@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(FT_ROWS *FT_COLS) k_server_frames(const FrameD
             } else {
                 const double cc = m ? d.p.c2 : d.p.c2b;
                 float f = fp.fade ? ff.fade : 1.f;
-                if (fp.fade_in_obstacle) f *= powf((float)cc / (float)d.p.c2, 0.1f);
+                if (fp.fade_in_obstacle) f *= powf(fade_ratio((float)cc, 1.f / (float)d.p.c2), 0.1f);
                 if (!colour_fast(lut, hue, f, 8e-7f, o)) frame_colour64(fp, lut, hue, 1.0, cc, d.p.c2, o);
             }
         }
