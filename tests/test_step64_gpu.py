@@ -4,6 +4,10 @@ every boundary rule, mask and table coefficients, and fields that the integer La
 refuses and mixes: noise, exponential tails over hundreds of binades, zeros of both signs,
 subnormals, infinities.  Scenes and batches must hold the oracle's values, the drop-in the
 oracle's bits."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -80,3 +84,43 @@ def test_scene_batch_and_dropin(bc, kind, kappa, gamma):
             got, nan = got.reshape(-1), np.isnan(w)
             assert np.array_equal(np.isnan(got), nan)
             assert np.array_equal(got[~nan].view(np.uint64), w[~nan].view(np.uint64)), (nx, ny, "drop-in")
+
+
+THREADS = """
+import sys, threading
+sys.path.insert(0, {tests!r})
+import conftest  # noqa: F401  (loads the package)
+import numpy as np
+from youtube_simulations_gb300 import params as P
+from youtube_simulations_gb300 import wavegpu as W
+
+CASES = [(P.FP64, 0.0, P.BC_DIRICHLET), (P.FP64, 1e-3, P.BC_ABSORBING), (P.FP32, 0.0, P.BC_DIRICHLET), (P.FP32, 1e-3, P.BC_PERIODIC)]
+
+def run(k, out):
+    prec, kappa, bc = CASES[k % len(CASES)]
+    p = P.make_params(150, 203, b_cond=bc, courant=0.3, kappa=kappa)
+    f = np.random.default_rng(k % len(CASES)).standard_normal(150 * 203)
+    with W.Scene(p, prec, P.COEF_MASK) as s:
+        if prec == P.FP32:
+            s.set_blocking(4, 16, 1)
+        s.upload(f, 0.9 * f, np.ones(150 * 203, np.int16))
+        for _ in range(5):
+            s.step(4)
+        out[k] = s.download()
+
+got, want = {{}}, {{}}
+threads = [threading.Thread(target=run, args=(k, got)) for k in range(12)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+[run(k, want) for k in range(12)]
+assert all(np.array_equal(a, b) for k in range(12) for a, b in zip(got[k], want[k]))
+print("same")
+"""
+
+
+def test_first_updates_from_several_threads():
+    """A process whose first updates come from several threads at once: what the launches ask of the device
+    and keep is the same whichever thread asks."""
+    here = Path(__file__).resolve().parent
+    r = subprocess.run([sys.executable, "-c", THREADS.format(tests=str(here))], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]

@@ -281,7 +281,7 @@ __global__ void k_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch)
 void launch_grid_ghosts(float *f0, float *f1, int nx, int ny, int pitch, cudaStream_t st)
 {
     const long long gt = BATCH_GHOST_COLS + BATCH_GHOST_COLS_R, total = gt * nx + 2LL * BATCH_GHOST_ROWS * (ny + gt);
-    k_grid_ghosts<<<(unsigned)std::min(608LL, (total + 127) / 128), 128, 0, st>>>(f0, f1, nx, ny, pitch);
+    k_grid_ghosts<<<(unsigned)std::min(4LL * sm_count(), (total + 127) / 128), 128, 0, st>>>(f0, f1, nx, ny, pitch);
 }
 
 // The ghost words and rows of a wrapped scene's active plane: one thread per word of rows

@@ -1,6 +1,7 @@
 // wg_internal.h — declarations shared by the library's translation units.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <string>
 #include "../../include/wavegpu.h"
 #include "wg_device.cuh"
@@ -96,6 +97,25 @@ template <class H> void launch_state_in32(int nx, int ny, int pitch, const H *ph
 // Fields (x0, y0), or (x1, y1) where *sel is not 0, to dense (phi, psi) rows; either may be NULL
 template <class T, class H> void launch_state_out(int nx, int ny, int pitch, const T *x0, const T *y0, const T *x1,
                                                   const T *y1, const int *sel, H *phi, H *psi, cudaStream_t st);
+// A positive number of each device (its SMs, a kernel's resident blocks), asked for once and kept.  Threads
+// that ask at the same time compute the same number.
+class PerDevice {
+    std::atomic<int> v_[16] = {};
+public:
+    template <class F> int get(const F &ask)
+    {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) return ask();
+        int n = v_[dev].load(std::memory_order_acquire);
+        if (n <= 0) {
+            n = ask();
+            v_[dev].store(n, std::memory_order_release);
+        }
+        return n;
+    }
+};
+int sm_count();  // SMs of the current device
+
 // The device address of n page-locked cells that kernels may access as H, or nullptr (rows that are
 // not aligned to their cells too: a copy takes any address, a kernel does not).
 template <class H> inline H *mapped_cells(H *p, size_t n)

@@ -23,6 +23,17 @@ namespace wg {
 // ---------------------------------------------------------------------------
 // FP64 updates (scenes and the drop-in)
 // ---------------------------------------------------------------------------
+int sm_count()
+{
+    static PerDevice sms;
+    return sms.get([] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return std::max(1, n);
+    });
+}
+
 // One update: blocks of boundary-line cells, then a warp per strip of ST_COLS columns and `rows`
 // rows (wg_step64.cuh).  3840x2160 two-medium table, GAMMA = 1e-4: 104 us an update
 // (80 Gcell/s, FP64 pipe 75% busy), 166 with every operation on the FP64 pipe and the edge lines
@@ -30,14 +41,13 @@ namespace wg {
 // registers (96 spill and measured 12% slower on tables).
 template <int COEF, bool EXACT, int Z>
 __global__ void __launch_bounds__(128, 4) k_step64(const __grid_constant__ DevParams p, const __grid_constant__ Strip64 a,
-                                                   int edge_blocks, int strips, int rows, long long time)
+                                                   int edge_blocks, int strips, int rows, bool few, long long time)
 {
     pdl_wait();  // launched by launch_pdl: the previous update has completed
-    // The next launch may come from here on where this one leaves most SMs free (fewer blocks than
+    // The next launch may come from here on where this one leaves SMs free (few: no more blocks than
     // SMs: 71x88, 4.1 to 3.8 us an update), otherwise after the work: its blocks, resident early, would
     // crowd the SMs that this one leaves first, and a launch of less than a wave that is bound by
     // the FP64 pipe would run at their rate (650x2026, an update and an energy: 294 us so, 171 now).
-    const bool few = gridDim.x <= 152;
     if (few) pdl_trigger();
     if ((int)blockIdx.x < edge_blocks) {  // a thread per boundary-line cell
         const int q = blockIdx.x * 128 + threadIdx.x;
@@ -54,14 +64,12 @@ __global__ void __launch_bounds__(128, 4) k_step64(const __grid_constant__ DevPa
 template <int COEF, bool EXACT, int Z>
 static void launch_step64_z(const DevParams &p, const Strip64 &a, long long time, cudaStream_t st)
 {
-    static int resident = 0;  // warps on the device
-    if (!resident) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    static PerDevice warps_on;
+    const int resident = warps_on.get([] {  // warps on the device
+        int per = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_step64<COEF, EXACT, Z>, 128, 0);
-        resident = std::max(1, sms) * std::max(1, per) * 4;
-    }
+        return sm_count() * std::max(1, per) * 4;
+    });
     // about three waves of warps: fewer leave SMs idle behind strips outside the domain, more
     // unpack too many rows twice (1280x720 ellipse, us an update by rows of a strip: 1: 12.0,
     // 2: 9.9, 3: 9.6 (chosen), 4: 10.1, 7: 10.9; 1920x1080 table: 3: 20.5, 5: 19.9 (chosen), 8: 20.6)
@@ -69,8 +77,9 @@ static void launch_step64_z(const DevParams &p, const Strip64 &a, long long time
     const int rows = (int)std::min(256LL, std::max(1LL, ((long long)(p.nx - 2) * strips + 3LL * resident - 1) / (3LL * resident)));
     const long long warps = (long long)strips * ((p.nx - 2 + rows - 1) / rows);
     const int edge_blocks = (edge64_cells(p) + 127) / 128;
-    launch_pdl(k_step64<COEF, EXACT, Z>, dim3((unsigned)(edge_blocks + (warps + 3) / 4)), dim3(128), 0, st, p, a, edge_blocks,
-               strips, rows, time);
+    const long long blocks = edge_blocks + (warps + 3) / 4;
+    launch_pdl(k_step64<COEF, EXACT, Z>, dim3((unsigned)blocks), dim3(128), 0, st, p, a, edge_blocks, strips, rows,
+               blocks <= sm_count(), time);
 }
 
 // wave_energy's stepper (wave_energy.c:662-913) on the half domain j < ny/2, with
@@ -783,7 +792,7 @@ template void launch_energy<double>(const DevParams &, const double *, const dou
 template <class T>
 void launch_count_nonfinite(int nx, int ny, int pitch, const T *a, unsigned long long *count, cudaStream_t st)
 {
-    k_count_nonfinite<T><<<4 * 152, 256, 0, st>>>(nx, ny, pitch, a, count);
+    k_count_nonfinite<T><<<4 * sm_count(), 256, 0, st>>>(nx, ny, pitch, a, count);
 }
 template void launch_count_nonfinite<float>(int, int, int, const float *, unsigned long long *, cudaStream_t);
 template void launch_count_nonfinite<double>(int, int, int, const double *, unsigned long long *, cudaStream_t);

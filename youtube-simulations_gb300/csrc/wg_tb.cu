@@ -938,31 +938,18 @@ static bool skew_shape_ok(const DevParams &p, int K, int S)
     return K >= 2 && K <= WG_SKEW_MAX_K && S >= 8 && S <= 4096 && p.ny >= 8 && p.nx >= 2;
 }
 
-static int sm_count()
-{
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 template <int COEF, int P, int PL, bool WRAP>
 static int skew_capacity()
 {
     const auto kernel = WRAP ? k_step_wrap<COEF, P, PL> : k_step_skew<COEF, P, PL>;
     constexpr size_t smem = SkewShm<COEF, PL, P>::BYTES;
-    static int per_sm = 0;
-    if (!per_sm) {
+    static PerDevice cap;
+    return cap.get([&] {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + SkewShm<COEF, PL, P>::OSC_BYTES));
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, 32 * P, smem);
-        per_sm = nb > 0 ? nb : 1;
-    }
-    return per_sm * sm_count();
+        return std::max(1, nb) * sm_count();
+    });
 }
 
 template <int COEF, int P, int PL>
@@ -1241,14 +1228,13 @@ template <int P, int PL>
 static int batch_skew_cap_p()
 {
     constexpr size_t smem = SkewShm<WG_COEF_MASK, PL, P>::BYTES;
-    static int per_sm = 0;
-    if (!per_sm) {
+    static PerDevice cap;
+    return cap.get([] {
         cudaFuncSetAttribute(k_batch_skew<P, PL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int nb = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_skew<P, PL>, 32 * P, smem);
-        per_sm = nb > 0 ? nb : 1;
-    }
-    return per_sm * sm_count();
+        return std::max(1, nb) * sm_count();
+    });
 }
 
 int batch_skew_form(const wg_params &p)
