@@ -54,3 +54,19 @@ def test_pipeline_equals_single_updates(form, coef):
         for k, rows in [(2, 8), (3, 8), (4, 8), (5, 8), (6, 8), (6, 64)]:
             got = run(p, coef, xy, phi, psi, tab, (k, rows, 1), n)
             assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (nx, ny, k, rows)
+
+
+@pytest.mark.parametrize("form", ["masked", "every", "masked_absorbing", "general", "osc"])
+@pytest.mark.parametrize("coef", [P.COEF_MASK, P.COEF_TABLE])
+def test_pipeline_near_the_stability_limit(form, coef):
+    """The same at a Courant number where a wrong value at the far end of a halo is not lost in rounding."""
+    for nx, ny in SIZES:
+        p, xy, phi, psi, _ = scene(form, nx, ny)
+        p.courant, p.courantb = 0.65, 0.5
+        tab = scenes.tables(p, xy)
+        n = 17
+        want = run(p, coef, xy, phi, psi, tab, (1,), n)
+        assert np.isfinite(want[0]).all()
+        for k, rows in [(2, 8), (3, 8), (4, 8), (5, 8), (6, 8), (6, 64)]:
+            got = run(p, coef, xy, phi, psi, tab, (k, rows, 1), n)
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (nx, ny, k, rows)

@@ -90,3 +90,39 @@ def test_laplacian_bits(lap, kind):
 def test_all_zero_cell(lap):
     out, ok = lap(np.zeros((1, 5)))
     assert ok[0] and out.view(np.uint64)[0] == 0
+
+
+SUB = r"""
+#include "wg_soft64.h"
+extern "C" void sub(long n, const double *v, double *out, unsigned char *ok)
+{
+    for (long i = 0; i < n; i++) {
+        bool k;
+        out[i] = wg::s64_sub(wg::s64_unpack(v[2 * i]), wg::s64_unpack(v[2 * i + 1]), k);
+        ok[i] = k;
+    }
+}
+"""
+
+
+@pytest.mark.parametrize("kind", ["uniform", "near", "nearer", "spread", "ties", "zeros", "special"])
+def test_difference_bits(tmp_path, kind):
+    """s64_sub: the bits of x - y wherever it accepts them."""
+    (tmp_path / "d.cpp").write_text(SUB)
+    subprocess.run(["g++", "-O2", "-shared", "-fPIC", "-ffp-contract=off", f"-I{CSRC}", "-o", str(tmp_path / "d.so"), str(tmp_path / "d.cpp")],
+                   check=True)
+    rng = np.random.default_rng(12)
+    v = np.ascontiguousarray(family(kind, 300_000, rng)[:, :2])
+    if kind == "nearer":  # neighbours in the last bits, and equal
+        v[:, 1] = v[:, 0] * (1.0 + 2.0 ** -52 * rng.integers(-6, 7, len(v)))
+    out, ok = np.empty(len(v)), np.empty(len(v), np.uint8)
+    ctypes.CDLL(str(tmp_path / "d.so")).sub(ctypes.c_long(len(v)), v.ctypes.data_as(ctypes.c_void_p), out.ctypes.data_as(ctypes.c_void_p),
+                                            ok.ctypes.data_as(ctypes.c_void_p))
+    ok = ok.astype(bool)
+    with np.errstate(all="ignore"):
+        want = v[:, 0] - v[:, 1]
+    assert np.array_equal(out[ok].view(np.uint64), want[ok].view(np.uint64))
+    if kind in ("uniform", "near", "ties"):
+        assert ok.mean() > 0.8
+    refused = ~np.isfinite(v).all(1) | (v.view(np.uint64) == np.uint64(1 << 63)).any(1) | ((v != 0) & (np.abs(v) < 2.3e-308)).any(1)
+    assert not ok[refused].any()
