@@ -255,3 +255,23 @@ def test_velocities_below_an_ulp_of_phi(plot, color_range):
             hv = palette_position(p, plot, x, y, xy, kw)
             diff = np.any(img != ref, axis=-1) & (np.abs(hv - np.round(hv)) >= 1e-11)
             assert not diff.any(), (int(diff.sum()), np.argwhere(diff)[:5])
+
+
+def test_log_energy_of_a_velocity_that_psi_loses():
+    """A flat FP32 field whose velocity is less than half an FP64 ulp of phi: the oracle's energy is 0, FP32's
+    is not, and they differ by far more than their logarithm's first-order error."""
+    nx, ny = 9, 40
+    n = nx * ny
+    p = P.make_params(nx, ny, b_cond=P.BC_DIRICHLET, courant=0.1, gamma=0.6, e_scale=1e6)
+    phi = np.full(n, float(np.float32(1e26)))
+    psi = phi - np.spacing(phi)
+    kw = dict(size=1, slope=1.0, scale=1.0, log_scale=2e-4, log_shift=0.0328, color_range=30.0)
+    L = np.repeat(np.arange(256), 3).reshape(256, 3).astype(np.uint8)
+    with W.Scene(p, P.FP32, P.COEF_MASK) as s:
+        s.set_blocking(1)
+        s.upload(phi, psi, np.ones(n, np.int16))
+        s.step(1)
+        img = s.frame_rgb8(L, plot=4, **kw)
+        x, y = s.download()
+    assert np.array_equal(x, y)
+    assert np.array_equal(img, oracle.frame_rgb8(p, x, np.ones(n), L, plot=4, psi=y, **kw))

@@ -108,11 +108,13 @@ __device__ __noinline__ int frame_hue_flux(const wg_frame_params &fp, double mgx
 }
 
 // value +- err of the modes that need no FP64: LOG_SHIFT + LOG_SCALE*log(q) of q with relative
-// error rel and absolute error tiny
+// error rel and absolute error tiny (FP64 where that is more than half of q: |log(1 - t)| is below
+// 2t, the factor hue_fast takes, only for smaller t)
 __device__ __forceinline__ float log_fast(const FrameFast &f, float q, float rel, float tiny, float *err)
 {
     const float l = logf(q);
     *err = fabsf(f.log_scale) * (rel + tiny / q + 5e-7f * fabsf(l) + 2e-7f) + 3e-7f * (fabsf(f.log_shift) + fabsf(f.log_scale * l));
+    if (!(tiny <= 0.5f * q)) *err = INFINITY;
     return f.log_shift + f.log_scale * l;
 }
 
