@@ -119,7 +119,8 @@ static __device__ __noinline__ void frame_colour64(const wg_frame_params &fp, co
                                                    double cc, double c2, uint8_t *o)
 {
     double f = dim;
-    if (fp.fade_in_obstacle) f *= pow(cc / c2, 0.1);  // (NaN, and so black, where COURANT = 0 makes it 0/0)
+    // (1 where cc is c2; NaN, and so black, where COURANT = 0 makes it 0/0)
+    if (fp.fade_in_obstacle && !(cc == c2 && c2 > 0.0 && c2 < INFINITY)) f *= pow(cc / c2, 0.1);
     if (fp.fade) f *= fp.fade_value;
     for (int q = 0; q < 3; q++) {
         const double v = (double)lut[hue * 3 + q] * f;
