@@ -12,6 +12,7 @@
 // factors, other cells black.  The reference hands floats to glColor3f; here the
 // palette is the caller's byte table and the faded colour is rounded to bytes.
 #include <cmath>
+#include <type_traits>
 #include "wg_internal.h"
 #include "wg_frame.cuh"
 #include "wg_scene.h"
@@ -120,16 +121,16 @@ __device__ __forceinline__ float log_fast(const FrameFast &f, float q, float rel
 
 // One block per tile of pixels, a thread per pixel.  The running sums (acc) are kept column by
 // column (k = col*h + row), as they are read.
-template <class T, int COEF>
-__global__ void __launch_bounds__(FT_ROWS *FT_COLS) k_frame_rgb8(const __grid_constant__ DevParams p, const T *__restrict__ phi,
+template <class T, int COEF, int COLS>
+__global__ void __launch_bounds__(FT_ROWS *COLS, COLS == FT_COLS_FLUX ? 16 : 1) k_frame_rgb8(const __grid_constant__ DevParams p, const T *__restrict__ phi,
                                                        const T *__restrict__ psi, const uint32_t *__restrict__ nz,
                                                        const T *__restrict__ tcc, const uint8_t *__restrict__ lut,
                                                        const __grid_constant__ wg_frame_params fp,
                                                        const __grid_constant__ FrameFast ff, double *__restrict__ acc,
                                                        uint8_t *__restrict__ out, int w, int h)
 {
-    __shared__ FrameTile sh;
-    const int row = blockIdx.y * FT_ROWS + threadIdx.x, col = blockIdx.x * FT_COLS + threadIdx.y;
+    __shared__ FrameTile<COLS> sh;
+    const int row = blockIdx.y * FT_ROWS + threadIdx.x, col = blockIdx.x * COLS + threadIdx.y;
     if (col < w && row < h) {
         const int i = col * fp.size, j = row * fp.size, plot = fp.plot;
         uint8_t *o = &sh.c[threadIdx.x][3 * threadIdx.y];
@@ -248,17 +249,18 @@ wg_status frame_launch(const DevParams &p, const void *phi, const void *psi, int
 {
     const int w = p.nx / fp.size, h = p.ny / fp.size;
     const FrameFast ff = frame_fast(fp, p);
-    const dim3 grd(frame_tiles_x(w), frame_tiles_y(h)), blk(FT_ROWS, FT_COLS);
-    const auto go = [&](auto kernel, auto *x, auto *y, auto *t) { kernel<<<grd, blk, 0, st>>>(p, x, y, nz, t, lut, fp, ff, acc, out, w, h); };
-    if (prec == WG_FP32) {
-        const float *x = (const float *)phi, *y = (const float *)psi, *t = (const float *)tcc;
-        if (coef == WG_COEF_TABLE) go(k_frame_rgb8<float, WG_COEF_TABLE>, x, y, t);
-        else go(k_frame_rgb8<float, WG_COEF_MASK>, x, y, t);
-    } else {
-        const double *x = (const double *)phi, *y = (const double *)psi, *t = (const double *)tcc;
-        if (coef == WG_COEF_TABLE) go(k_frame_rgb8<double, WG_COEF_TABLE>, x, y, t);
-        else go(k_frame_rgb8<double, WG_COEF_MASK>, x, y, t);
-    }
+    const auto go = [&](auto cols, auto *x, auto *y, auto *t) {
+        using T = std::remove_cv_t<std::remove_pointer_t<decltype(x)>>;
+        constexpr int COLS = decltype(cols)::value;
+        const auto kernel = coef == WG_COEF_TABLE ? k_frame_rgb8<T, WG_COEF_TABLE, COLS> : k_frame_rgb8<T, WG_COEF_MASK, COLS>;
+        kernel<<<dim3(frame_tiles_x(w, COLS), frame_tiles_y(h)), dim3(FT_ROWS, COLS), 0, st>>>(p, x, y, nz, t, lut, fp, ff, acc, out, w, h);
+    };
+    const auto tiled = [&](auto *x, auto *y, auto *t) {
+        if (fp.plot == WG_P_TOTAL_ENERGY_FLUX) go(std::integral_constant<int, FT_COLS_FLUX>(), x, y, t);
+        else go(std::integral_constant<int, FT_COLS>(), x, y, t);
+    };
+    if (prec == WG_FP32) tiled((const float *)phi, (const float *)psi, (const float *)tcc);
+    else tiled((const double *)phi, (const double *)psi, (const double *)tcc);
     WG_CUDA(cudaGetLastError());
     return WG_OK;
 }

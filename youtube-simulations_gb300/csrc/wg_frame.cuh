@@ -15,11 +15,14 @@
 
 namespace wg {
 
-// A block renders FT_ROWS x FT_COLS pixels: a warp reads FT_ROWS frame rows of one column i
+// A block renders FT_ROWS x COLS pixels: a warp reads FT_ROWS frame rows of one column i
 // (contiguous along j), and the colours go to the frame through shared memory, row by row.
-// (32 columns a block measured the same on large frames and twice as slow on a 64x32 one.)
-constexpr int FT_ROWS = 32, FT_COLS = 8;
-__host__ __device__ inline int frame_tiles_x(int w) { return (w + FT_COLS - 1) / FT_COLS; }
+// FT_COLS columns (32 columns a block measured the same on large frames and twice as slow on a 64x32
+// one); half as many for the total flux, whose pixels are FP64 throughout and a chain: blocks that fit
+// the SMs all at once, 32 registers a thread, and divide among them more evenly (1280x720 at size 2,
+// 48 registers and 8 columns: 81 us; now 71 to 72, and 69 with a thread per pixel along i before).
+constexpr int FT_ROWS = 32, FT_COLS = 8, FT_COLS_FLUX = 4;
+__host__ __device__ inline int frame_tiles_x(int w, int cols = FT_COLS) { return (w + cols - 1) / cols; }
 __host__ __device__ inline int frame_tiles_y(int h) { return (h + FT_ROWS - 1) / FT_ROWS; }
 
 struct FrameFast {
@@ -131,17 +134,19 @@ static __device__ __noinline__ void frame_colour64(const wg_frame_params &fp, co
 
 // The block's colours, sh[row][3*col..], to the frame (w x h pixels, tile (tx, ty)); call after a
 // barrier.
+template <int COLS>
 struct FrameTile {
-    uint8_t c[FT_ROWS][3 * FT_COLS + 4];
+    uint8_t c[FT_ROWS][3 * COLS + 4];
 };
-__device__ __forceinline__ void frame_tile_out(const FrameTile &sh, uint8_t *out, int w, int h, int tx, int ty)
+template <int COLS>
+__device__ __forceinline__ void frame_tile_out(const FrameTile<COLS> &sh, uint8_t *out, int w, int h, int tx, int ty)
 {
-    const int n = 3 * min(FT_COLS, w - tx * FT_COLS), rows = min(FT_ROWS, h - ty * FT_ROWS);
+    const int n = 3 * min(COLS, w - tx * COLS), rows = min(FT_ROWS, h - ty * FT_ROWS);
     const int t = threadIdx.y * FT_ROWS + threadIdx.x;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const int q = t + k * FT_ROWS * FT_COLS, row = q / (3 * FT_COLS), b = q - row * 3 * FT_COLS;
-        if (row < rows && b < n) out[((size_t)(ty * FT_ROWS + row) * w + (size_t)tx * FT_COLS) * 3 + b] = sh.c[row][b];
+        const int q = t + k * FT_ROWS * COLS, row = q / (3 * COLS), b = q - row * 3 * COLS;
+        if (row < rows && b < n) out[((size_t)(ty * FT_ROWS + row) * w + (size_t)tx * COLS) * 3 + b] = sh.c[row][b];
     }
 }
 

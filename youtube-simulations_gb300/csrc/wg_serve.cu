@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(FT_ROWS *FT_COLS) k_server_frames(const FrameD
                                                           const __grid_constant__ wg_frame_params fp,
                                                           const __grid_constant__ FrameFast ff, uint8_t *__restrict__ out)
 {
-    __shared__ FrameTile sh;
+    __shared__ FrameTile<FT_COLS> sh;
     int lo = 0, hi = ntab - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
