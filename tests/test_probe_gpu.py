@@ -65,3 +65,24 @@ def test_dropin_resident_cell():
     for i, j in [(5, 7), (30, 20), (66, 44)]:
         assert W.dropin_cell(rf, i, j) == new.reshape(p.nx, p.ny)[i, j]
     W.set_mode(False)
+
+
+@pytest.mark.parametrize("bc", [P.BC_PERIODIC, P.BC_DIRICHLET])
+def test_probes_set_before_the_first_step(bc):
+    """The first step of a size class times candidate blockings; the probes sample none of those updates."""
+    nx, ny = 1100, 9 if bc == P.BC_PERIODIC else 17
+    n = nx * ny
+    rng = np.random.default_rng(1)
+    p = P.make_params(nx, ny, b_cond=bc, courant=0.3)
+    phi, xy = rng.standard_normal(n), np.ones(n, np.int16)
+    cells = [(0, 0), (5, 3), (nx - 1, ny - 1)]
+    got = []
+    for blocking in (0, 1):
+        with W.Scene(p, P.FP32, P.COEF_MASK) as s:
+            if blocking:
+                s.set_blocking(1)
+            s.upload(phi, 0.9 * phi, xy)
+            s.set_probes(cells, capacity=4000)
+            s.step(7)
+            got.append(s.read_probes())
+    assert got[0].shape == (7, len(cells)) and np.array_equal(*got)

@@ -1566,6 +1566,8 @@ void autotune_scene(wg_scene *s)
         const long long t_save = s->time;
         const int cur_save = s->cur;
         void *const bufs[] = {s->f[0], s->f[1], s->g[0], s->g[1]};  // the fields return to their buffers
+        const int probes = s->probe_n;  // the probes sample the scene's updates, not these
+        s->probe_n = 0;
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
@@ -1606,6 +1608,7 @@ void autotune_scene(wg_scene *s)
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         s->cur = cur_save;
+        s->probe_n = probes;
         for (int k = 0; k < 2; k++) {
             s->f[k] = bufs[k];
             s->g[k] = bufs[2 + k];
