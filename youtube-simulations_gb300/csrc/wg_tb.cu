@@ -1625,6 +1625,7 @@ void autotune_scene(wg_scene *s)
     s->tb_k = best_k;
     s->tile_i = best_l;
     s->tile_j = best_w;
+    if (!ok) return;  // no memory for the copy: single updates for this scene, but not for its class
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune[key] = {best_k, best_l, best_w};
 }
