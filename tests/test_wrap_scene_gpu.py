@@ -225,3 +225,22 @@ def test_upload_that_fails_half_way():
             out.append(s.download(native=True))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_calls_of_two_updates():
+    """Calls of 2 updates take single updates, beside calls that take passes."""
+    nx, ny = 45, 225
+    n = nx * ny
+    rng = np.random.default_rng(11)
+    p = P.make_params(nx, ny, b_cond=P.BC_PERIODIC, courant=0.6)
+    f = rng.standard_normal(n), rng.standard_normal(n), (rng.random(n) < 0.9).astype(np.int16)
+    out = []
+    for blocking in [(1,), (6, 8, 1), (2, 8, 1)]:
+        with W.Scene(p, P.FP32, P.COEF_MASK) as s:
+            s.upload(*f)
+            s.set_blocking(*blocking)
+            for k in (2, 6, 2, 2, 4, 3, 2, 1, 2, 12):
+                s.step(k)
+            out.append(s.download(native=True))
+    for got in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(got, out[0]))

@@ -254,8 +254,12 @@ wg_status scene_step_impl(wg_scene *s, int nsteps)
     if (wg_status st = scene_recording(s, &rec)) return st;
     if (s->recorded) s->ghosts_ok = false;
     if (rec) s->mask_ghosts_ok = false;
-    // probes sample every update; the TMA tiles do not wrap
-    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1);
+    // probes sample every update; the TMA tiles do not wrap.  A periodic grid's two updates are faster
+    // as such than as a pass of one-warp teams, which also write its ghosts, up to about 2560x1440 (us
+    // a call, updates / pass: 256x192 9.3 / 14.8, 1277x717 13.4 / 18.3, 2560x1440 22.4 / 23.2 or,
+    // with tables, 25.1 / 24.7, 3840x2160 47 / 36)
+    const bool two = s->wrap && nsteps == 2 && (long long)s->prm.nx * s->prm.ny < (1LL << 22);
+    const bool tb = k > 1 && tb_supported(s) && !s->probe_n && !(s->wrap && s->tile_j != 1) && !two;
     if (tb) {
         wg_status st = tb_prepare(s, nsteps);
         if (st) return st;
