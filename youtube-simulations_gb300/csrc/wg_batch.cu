@@ -1031,22 +1031,25 @@ wg_status wg_batch_download(wg_batch *b, int32_t slot, double *phi, double *psi)
     // state, a second wait and a stage each time: 1277x717 114 to 88 us, grids of 240x240 about
     // 41 to 14 us.)
     double *stage = nullptr, *ophi = phi, *opsi = psi;
+    const size_t m = state_stage_cells(n);
     const bool mapped = mapped_rows(ophi, opsi, n);
     if (!mapped) {
-        WG_CUDA(cudaMallocAsync((void **)&stage, 2 * n * sizeof(double), b->st));
+        WG_CUDA(cudaMallocAsync((void **)&stage, 2 * m * sizeof(double), b->st));
         ophi = phi ? stage : nullptr;
-        opsi = psi ? stage + n : nullptr;
+        opsi = psi ? stage + m : nullptr;
     }
     if (b->prec == WG_FP32) {  // phi, and psi = phi - v
-        launch_state_out<float, double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const float *)h.f[0], (const float *)h.f[1],
-                                        (const float *)h.f[2], (const float *)h.f[3], &b->d_dyn[slot].pair, ophi, opsi, b->st);
+        const auto launch = mapped ? launch_state_out<float, double> : launch_state_stage<float, double>;
+        launch(h.prm.nx, h.prm.ny, h.dp.pitch, (const float *)h.f[0], (const float *)h.f[1], (const float *)h.f[2],
+               (const float *)h.f[3], &b->d_dyn[slot].pair, ophi, opsi, b->st);
     } else {
-        launch_state_out<double, double>(h.prm.nx, h.prm.ny, h.dp.pitch, (const double *)h.f[0], (const double *)h.f[1],
-                                         (const double *)h.f[1], (const double *)h.f[0], &b->d_dyn[slot].cur, ophi, opsi, b->st);
+        const auto launch = mapped ? launch_state_out<double, double> : launch_state_stage<double, double>;
+        launch(h.prm.nx, h.prm.ny, h.dp.pitch, (const double *)h.f[0], (const double *)h.f[1], (const double *)h.f[1],
+               (const double *)h.f[0], &b->d_dyn[slot].cur, ophi, opsi, b->st);
     }
     if (!mapped) {
         if (phi) WG_CUDA(cudaMemcpyAsync(phi, stage, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
-        if (psi) WG_CUDA(cudaMemcpyAsync(psi, stage + n, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
+        if (psi) WG_CUDA(cudaMemcpyAsync(psi, stage + m, n * sizeof(double), cudaMemcpyDeviceToHost, b->st));
         WG_CUDA(cudaFreeAsync(stage, b->st));
     }
     WG_CUDA(cudaGetLastError());

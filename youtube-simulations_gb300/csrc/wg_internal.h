@@ -97,6 +97,10 @@ template <class H> void launch_state_in32(int nx, int ny, int pitch, const H *ph
 // Fields (x0, y0), or (x1, y1) where *sel is not 0, to dense (phi, psi) rows; either may be NULL
 template <class T, class H> void launch_state_out(int nx, int ny, int pitch, const T *x0, const T *y0, const T *x1,
                                                   const T *y1, const int *sel, H *phi, H *psi, cudaStream_t st);
+// The same into a stage of device memory: phi and psi on 16 bytes, state_stage_cells(n) cells each
+template <class T, class H> void launch_state_stage(int nx, int ny, int pitch, const T *x0, const T *y0, const T *x1,
+                                                    const T *y1, const int *sel, H *phi, H *psi, cudaStream_t st);
+inline size_t state_stage_cells(size_t n) { return (n + 3) & ~(size_t)3; }
 // A positive number of each device (its SMs, a kernel's resident blocks), asked for once and kept.  Threads
 // that ask at the same time compute the same number.
 class PerDevice {

@@ -158,13 +158,14 @@ static wg_status download_state(wg_scene *s, H *phi, H *psi)
         if (phi) WG_CUDA(cudaMemcpy2DAsync(phi, ny * sizeof(H), x, s->pitch * sizeof(T), ny * sizeof(H), nx, cudaMemcpyDeviceToHost, s->st));
         if (psi) WG_CUDA(cudaMemcpy2DAsync(psi, ny * sizeof(H), y, s->pitch * sizeof(T), ny * sizeof(H), nx, cudaMemcpyDeviceToHost, s->st));
     } else {
-        if ((st = scene_alloc_dense_stage(s, 2 * bytes))) return st;
+        const size_t m = state_stage_cells(n);
+        if ((st = scene_alloc_dense_stage(s, 2 * m * sizeof(H)))) return st;
         H *stage = (H *)s->dstage;
-        launch_state_out<T, H>(nx, ny, s->pitch, x, y, x, y, nullptr, phi ? stage : nullptr, psi ? stage + n : nullptr, s->st);
+        launch_state_stage<T, H>(nx, ny, s->pitch, x, y, x, y, nullptr, phi ? stage : nullptr, psi ? stage + m : nullptr, s->st);
         s->launches++;
         WG_CUDA(cudaGetLastError());
         if (phi) WG_CUDA(cudaMemcpyAsync(phi, stage, bytes, cudaMemcpyDeviceToHost, s->st));
-        if (psi) WG_CUDA(cudaMemcpyAsync(psi, stage + n, bytes, cudaMemcpyDeviceToHost, s->st));
+        if (psi) WG_CUDA(cudaMemcpyAsync(psi, stage + m, bytes, cudaMemcpyDeviceToHost, s->st));
     }
     if ((st = flag_copy(s))) return st;
     WG_CUDA(cudaStreamSynchronize(s->st));
