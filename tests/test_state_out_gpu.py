@@ -80,3 +80,19 @@ def test_page_locked_rows_not_aligned_to_their_cells(prec, native, shift):
             b.step(3)
             W.check(W.lib().wg_batch_download(b.h, slot, rows[0].ctypes.data, rows[1].ctypes.data))
             assert all(np.array_equal(r.copy().view(dt), w) for r, w in zip(rows, b.download(slot)))
+
+
+@pytest.mark.parametrize("nx,ny", [(2045, 2049), (2050, 2053)])
+def test_fp64_rows_below_and_above_the_in_place_size(nx, ny):
+    """FP64 rows of less than 32 MB are copied, larger page-locked ones written in place."""
+    n = nx * ny
+    f = np.random.default_rng(1).standard_normal(n)
+    rows = [pinned(n, o, torch.float64) for o in (1, 3)]
+    with W.Scene(P.make_params(nx, ny, courant=0.1), P.FP64, P.COEF_MASK) as s:
+        s.upload(f, 0.5 * f, np.ones(n, np.int16))
+        s.step(1)
+        ref = s.download()
+        W.check(W.lib().wg_scene_download(s.h, rows[0][0].ctypes.data, rows[1][0].ctypes.data, P.FP64))
+    for (r, whole), o, want in zip(rows, (1, 3), ref):
+        assert np.array_equal(r, want)
+        assert np.all(whole[:o] == 7.0) and np.all(whole[o + n:] == 7.0)
