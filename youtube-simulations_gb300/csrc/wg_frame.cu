@@ -122,7 +122,7 @@ __device__ __forceinline__ float log_fast(const FrameFast &f, float q, float rel
 // One block per tile of pixels, a thread per pixel.  The running sums (acc) are kept column by
 // column (k = col*h + row), as they are read.
 template <class T, int COEF, int COLS>
-__global__ void __launch_bounds__(FT_ROWS *COLS, COLS == FT_COLS_FLUX ? 16 : 1) k_frame_rgb8(const __grid_constant__ DevParams p, const T *__restrict__ phi,
+__global__ void __launch_bounds__(FT_ROWS *COLS, COLS == FT_COLS_FLUX ? 16 : 0) k_frame_rgb8(const __grid_constant__ DevParams p, const T *__restrict__ phi,
                                                        const T *__restrict__ psi, const uint32_t *__restrict__ nz,
                                                        const T *__restrict__ tcc, const uint8_t *__restrict__ lut,
                                                        const __grid_constant__ wg_frame_params fp,
